@@ -363,7 +363,7 @@ struct GemmArgs {
     const __nv_bfloat16 *B;
     int lda, ldb, M, N, K;
     const float *bias;
-    int act;
+    int act;                    // 0 identity, 1 GELU, 2 times GELU'(Zin) (backward)
     float alpha, beta;
     float *C32;
     int ldc32;
@@ -372,7 +372,19 @@ struct GemmArgs {
     float *Z32;
     int ldz;
     int *err;
+    // operand given transposed: A as [K][lda] with M contiguous (readable up to
+    // M rounded up to 8), B as [K][ldb] with N contiguous
+    bool a_t, b_t;
+    const float *Zin;           // act 2: pre-activations, row stride ldz
+};
+// column sums of an FP32 [rows][ld] array, rows added in order
+struct ColSum {
+    const float *in;
+    int rows, cols, ld;
+    float *out;
 };
 bool gemm_bf16_launch(const GemmArgs &a, cudaStream_t st);
+// up to two independent GEMMs and one column sum in one launch (g1, cs may be null)
+bool gemm_bf16_group(const GemmArgs &g0, const GemmArgs *g1, const ColSum *cs, cudaStream_t st);
 
 }  // namespace fdtd

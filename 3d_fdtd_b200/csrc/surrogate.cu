@@ -6,16 +6,17 @@
 // alone); its CPU FP64 restatement is oracle/surrogate.py.
 //
 // Layout: layer l maps in_l -> out_l; W_l is stored [out_l][in_pad_l] (FP32
-// master and BF16 copy, K-major for the forward GEMM) and transposed
-// [in_pad_l][out_pad_l] in BF16 for the backward GEMM; padded columns are zero
-// and stay zero (the padded inputs are zero, so their gradients are).
+// master and BF16 copy; the backward GEMM reads the copy transposed); padded
+// columns are zero and stay zero (the padded inputs are zero, so their
+// gradients are).
 // Forward: Z_l = H_{l-1} W_l^T + b_l (FP32, kept), H_l = bf16(GELU(Z_l)),
 // Y = H_3 W_4^T + b_4 (FP32).  Loss: mean over batch and outputs of (Y-T)^2.
 // Backward per layer: db = column sums of dZ (FP32), dW = dZ^T H_{l-1}
-// (GEMM over the batch, both operands transposed to K-major BF16),
-// dH_{l-1} = dZ W_l, dZ_{l-1} = dH_{l-1} GELU'(Z_{l-1}); dX = dZ_1 W_1 for the
-// input gradient.  Rounding points (BF16 operands of every GEMM) are the ones
+// (GEMM over the batch, both operands read transposed), dH_{l-1} = dZ W_l,
+// dZ_{l-1} = dH_{l-1} GELU'(Z_{l-1}) in its epilogue; dX = dZ_1 W_1 for the
+// input gradient.  All of a layer's backward is one launch.  Rounding points (BF16 operands of every GEMM) are the ones
 // the restatement reproduces.
+#include <algorithm>
 #include <cmath>
 #include <cuda_bf16.h>
 #include <mutex>
@@ -32,16 +33,11 @@ constexpr int kLayers = 4;
 
 int pad8(int x) { return (x + 7) / 8 * 8; }
 
-__device__ __forceinline__ float gelu_grad(float x)
-{
-    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-    const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-    return cdf + x * pdf;
-}
-
 // f32 [rows][cols] -> bf16 [rows][ldo] (columns cols..ldo-1 zero)
 __global__ void k_pack_bf16(const float *in, int rows, int cols, int ldi, __nv_bfloat16 *out, int ldo)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long long n = (long long)rows * ldo;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const int r = (int)(t / ldo), c = (int)(t % ldo);
@@ -49,33 +45,12 @@ __global__ void k_pack_bf16(const float *in, int rows, int cols, int ldi, __nv_b
     }
 }
 
-// bf16 [rows][ld_in] (cols used) -> bf16 [cols_pad][ld_out] transposed (rows -> columns), zero padded
-__global__ void k_transpose_bf16(const __nv_bfloat16 *in, int rows, int cols, int ldi, __nv_bfloat16 *out,
-                                 int cols_pad, int ldo)
-{
-    const long long n = (long long)cols_pad * ldo;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(t / ldo), r = (int)(t % ldo);
-        out[t] = (c < cols && r < rows) ? in[(long long)r * ldi + c] : __float2bfloat16_rn(0.0f);
-    }
-}
-
-// f32 master W [out][inp] -> bf16 W [out][inp] and W^T [inp][outp]
-__global__ void k_cast_weights(const float *W, int out, int inp, int outp, __nv_bfloat16 *Wb, __nv_bfloat16 *WbT)
-{
-    const long long n = (long long)inp * outp;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / outp), o = (int)(t % outp);
-        const __nv_bfloat16 v = __float2bfloat16_rn(o < out ? W[(long long)o * inp + i] : 0.0f);
-        WbT[t] = v;
-        if (o < out) Wb[(long long)o * inp + i] = v;
-    }
-}
-
 // dZ = 2 (Y - T) / (B n) (f32 [B][n] and bf16 [B][np]); loss += sum (Y-T)^2 / (B n)
 __global__ void k_mse(const float *Y, const float *T, int B, int n, int np, float *dZ, __nv_bfloat16 *dZb,
                       double *loss)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long long cnt = (long long)B * np;
     const float s = 2.0f / ((float)B * (float)n);
     double acc = 0.0;
@@ -97,6 +72,8 @@ __global__ void k_mse(const float *Y, const float *T, int B, int n, int np, floa
 // given dY directly: dZ (f32 [B][n]) and bf16 [B][np]
 __global__ void k_seed_grad(const float *dy, int B, int n, int np, float *dZ, __nv_bfloat16 *dZb)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long long cnt = (long long)B * np;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cnt; t += (long long)gridDim.x * blockDim.x) {
         const int r = (int)(t / np), c = (int)(t % np);
@@ -106,37 +83,50 @@ __global__ void k_seed_grad(const float *dy, int B, int n, int np, float *dZ, __
     }
 }
 
-// dZ = dH * GELU'(Z): f32 [B][n] and bf16 [B][n]
-__global__ void k_gelu_back(const float *dH, const float *Z, long long cnt, float *dZ, __nv_bfloat16 *dZb)
+// Adam on every parameter of the network and the BF16 copy of them, in one
+// launch over the contiguous parameter buffers (n a multiple of 4; padding has
+// zero gradients and stays zero)
+__global__ void k_adam(float4 *p, const float4 *g, float4 *m, float4 *v, __nv_bfloat162 *pb, long long n4, float lr,
+                       float b1, float b2, float eps, float c1, float c2)
 {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cnt; t += (long long)gridDim.x * blockDim.x) {
-        const float g = dH[t] * gelu_grad(Z[t]);
-        dZ[t] = g;
-        dZb[t] = __float2bfloat16_rn(g);
-    }
-}
-
-// db[c] = sum_r dZ[r][c], one thread per column, rows in order
-__global__ void k_col_sum(const float *dZ, int B, int n, float *db)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    float s = 0.0f;
-    for (int r = 0; r < B; r++) s += dZ[(long long)r * n + c];
-    db[c] = s;
-}
-
-__global__ void k_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2,
-                       float eps, float c1, float c2)
-{
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const float gt = g[t];
-        const float mt = b1 * m[t] + (1.0f - b1) * gt;
-        const float vt = b2 * v[t] + (1.0f - b2) * gt * gt;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    auto upd = [&](float &pt, float gt, float &mt, float &vt) {
+        mt = b1 * mt + (1.0f - b1) * gt;
+        vt = b2 * vt + (1.0f - b2) * gt * gt;
+        pt -= lr * (mt / c1) / (sqrtf(vt / c2) + eps);
+    };
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n4; t += (long long)gridDim.x * blockDim.x) {
+        float4 pt = p[t], mt = m[t], vt = v[t];
+        const float4 gt = g[t];
+        upd(pt.x, gt.x, mt.x, vt.x);
+        upd(pt.y, gt.y, mt.y, vt.y);
+        upd(pt.z, gt.z, mt.z, vt.z);
+        upd(pt.w, gt.w, mt.w, vt.w);
+        p[t] = pt;
         m[t] = mt;
         v[t] = vt;
-        p[t] -= lr * (mt / c1) / (sqrtf(vt / c2) + eps);
+        pb[2 * t] = __nv_bfloat162(__float2bfloat16_rn(pt.x), __float2bfloat16_rn(pt.y));
+        pb[2 * t + 1] = __nv_bfloat162(__float2bfloat16_rn(pt.z), __float2bfloat16_rn(pt.w));
     }
+}
+
+// launch with a programmatic dependency on the preceding kernel of the stream:
+// every kernel here waits for it (griddepcontrol.wait) before it touches memory
+template <typename... P, typename... A>
+bool launch_chained(void (*k)(P...), int blocks, cudaStream_t st, A... args)
+{
+    note_launch();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_ok(cudaLaunchKernelEx(&cfg, k, P(args)...), "surrogate launch");
 }
 
 int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 2368); }
@@ -144,16 +134,21 @@ int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 2
 struct Mlp {
     int nin = 0, hid = 0, nout = 0;
     int in[kLayers], inp[kLayers], out[kLayers], outp[kLayers];
+    // parameters, gradients, Adam moments and the BF16 copy: one buffer each,
+    // layer after layer W [outp][inp] (rows out.. and columns in.. zero), then b [outp]
+    float *P = nullptr, *G = nullptr, *Mo = nullptr, *Vo = nullptr;
+    __nv_bfloat16 *Pb = nullptr;
+    long long total = 0;                     // elements of each, a multiple of 8
     float *W[kLayers] = {}, *b[kLayers] = {}, *gW[kLayers] = {}, *gb[kLayers] = {};
-    float *mW[kLayers] = {}, *vW[kLayers] = {}, *mb[kLayers] = {}, *vb[kLayers] = {};
-    __nv_bfloat16 *Wb[kLayers] = {}, *WbT[kLayers] = {};
+    __nv_bfloat16 *Wb[kLayers] = {};
     int step = 0;
     int cap = 0;
     float *xs = nullptr, *ts = nullptr, *dys = nullptr;   // f32 staging [cap][nin], [cap][nout]
-    __nv_bfloat16 *X = nullptr, *XT = nullptr;
-    __nv_bfloat16 *H[kLayers] = {}, *HT[kLayers] = {};
-    float *Z[kLayers] = {}, *Y = nullptr, *dZf = nullptr, *dH = nullptr, *dX = nullptr;
-    __nv_bfloat16 *dZb = nullptr, *dZbT = nullptr;
+    __nv_bfloat16 *X = nullptr;
+    __nv_bfloat16 *H[kLayers] = {};
+    float *Z[kLayers] = {}, *Y = nullptr, *dX = nullptr;
+    float *dZf[2] = {};                      // dZ of a layer, FP32 and BF16; layers alternate
+    __nv_bfloat16 *dZb[2] = {};
     double *loss = nullptr;
     int *err = nullptr;
     cudaStream_t st = nullptr;
@@ -173,7 +168,10 @@ struct Mlp {
         for (void *p : allocs) cudaFree(p);
         if (st) cudaStreamDestroy(st);
     }
-    long long wcount(int l) const { return (long long)out[l] * inp[l]; }
+    long long wcount(int l) const { return (long long)outp[l] * inp[l]; }
+    // host image of a parameter buffer <-> flat order W1 [out][in], b1, ..., unpadded
+    void flatten(const float *img, float *flat) const;
+    void unflatten(const float *flat, float *img) const;
     long long params() const
     {
         long long n = 0;
@@ -181,6 +179,26 @@ struct Mlp {
         return n;
     }
 };
+
+void Mlp::flatten(const float *img, float *flat) const
+{
+    for (int l = 0; l < kLayers; l++) {
+        const float *w = img + (W[l] - P), *bb = img + (b[l] - P);
+        for (int o = 0; o < out[l]; o++, flat += in[l]) std::copy(w + (size_t)o * inp[l], w + (size_t)o * inp[l] + in[l], flat);
+        flat = std::copy(bb, bb + out[l], flat);
+    }
+}
+
+void Mlp::unflatten(const float *flat, float *img) const
+{
+    std::fill(img, img + total, 0.0f);
+    for (int l = 0; l < kLayers; l++) {
+        float *w = img + (W[l] - P);
+        for (int o = 0; o < out[l]; o++, flat += in[l]) std::copy(flat, flat + in[l], w + (size_t)o * inp[l]);
+        std::copy(flat, flat + out[l], img + (b[l] - P));
+        flat += out[l];
+    }
+}
 
 bool mlp_setup(Mlp &m, int nin, int hid, int nout, unsigned long long seed)
 {
@@ -190,14 +208,18 @@ bool mlp_setup(Mlp &m, int nin, int hid, int nout, unsigned long long seed)
         m.in[l] = ins[l]; m.inp[l] = pad8(ins[l]); m.out[l] = outs[l]; m.outp[l] = pad8(outs[l]);
     }
     if (!cuda_ok(cudaStreamCreateWithFlags(&m.st, cudaStreamNonBlocking), "stream")) return false;
-    if (!m.alloc(&m.loss, 1) || !m.alloc(&m.err, 1)) return false;
+    if (!m.alloc(&m.loss, 2)) return false;
+    m.err = (int *)(m.loss + 1);             // read back together
+    for (int l = 0; l < kLayers; l++) m.total += m.wcount(l) + m.outp[l];
+    if (!m.alloc(&m.P, m.total) || !m.alloc(&m.G, m.total) || !m.alloc(&m.Mo, m.total) || !m.alloc(&m.Vo, m.total) ||
+        !m.alloc(&m.Pb, m.total))
+        return false;
+    long long at = 0;
     for (int l = 0; l < kLayers; l++) {
-        const long long nw = m.wcount(l);
-        if (!m.alloc(&m.W[l], nw) || !m.alloc(&m.gW[l], nw) || !m.alloc(&m.mW[l], nw) || !m.alloc(&m.vW[l], nw) ||
-            !m.alloc(&m.b[l], m.out[l]) || !m.alloc(&m.gb[l], m.out[l]) || !m.alloc(&m.mb[l], m.out[l]) ||
-            !m.alloc(&m.vb[l], m.out[l]) || !m.alloc(&m.Wb[l], nw) ||
-            !m.alloc(&m.WbT[l], (size_t)m.inp[l] * m.outp[l]))
-            return false;
+        m.W[l] = m.P + at; m.gW[l] = m.G + at; m.Wb[l] = m.Pb + at;
+        at += m.wcount(l);
+        m.b[l] = m.P + at; m.gb[l] = m.G + at;
+        at += m.outp[l];
     }
     // PyTorch-Linear-like init: U(-1/sqrt(in), 1/sqrt(in)), seeded splitmix64
     unsigned long long s = seed;
@@ -209,30 +231,22 @@ bool mlp_setup(Mlp &m, int nin, int hid, int nout, unsigned long long seed)
         z ^= z >> 31;
         return (double)(z >> 11) * (1.0 / 9007199254740992.0);
     };
-    std::vector<float> hw, hb;
+    std::vector<float> flat, img((size_t)m.total);
     for (int l = 0; l < kLayers; l++) {
         const double bound = 1.0 / std::sqrt((double)m.in[l]);
-        hw.assign(m.wcount(l), 0.0f);
-        for (int o = 0; o < m.out[l]; o++)
-            for (int i = 0; i < m.in[l]; i++) hw[(size_t)o * m.inp[l] + i] = (float)((2 * uni() - 1) * bound);
-        hb.resize(m.out[l]);
-        for (auto &v : hb) v = (float)((2 * uni() - 1) * bound);
-        if (!cuda_ok(cudaMemcpyAsync(m.W[l], hw.data(), hw.size() * 4, cudaMemcpyHostToDevice, m.st), "init") ||
-            !cuda_ok(cudaMemcpyAsync(m.b[l], hb.data(), hb.size() * 4, cudaMemcpyHostToDevice, m.st), "init") ||
-            !cuda_ok(cudaStreamSynchronize(m.st), "init"))
-            return false;
+        for (int q = 0; q < m.out[l] * m.in[l] + m.out[l]; q++) flat.push_back((float)((2 * uni() - 1) * bound));
     }
+    m.unflatten(flat.data(), img.data());
+    if (!cuda_ok(cudaMemcpyAsync(m.P, img.data(), img.size() * sizeof(float), cudaMemcpyHostToDevice, m.st), "init") ||
+        !cuda_ok(cudaStreamSynchronize(m.st), "init"))
+        return false;
     return true;
 }
 
 bool refresh_bf16(Mlp &m)
 {
-    for (int l = 0; l < kLayers; l++) {
-        note_launch();
-        k_cast_weights<<<blocks_for((long long)m.inp[l] * m.outp[l]), 256, 0, m.st>>>(m.W[l], m.out[l], m.inp[l],
-                                                                                        m.outp[l], m.Wb[l], m.WbT[l]);
-    }
-    return cuda_ok(cudaGetLastError(), "cast weights");
+    const int row = 8;
+    return launch_chained(k_pack_bf16, blocks_for(m.total), m.st, m.P, (int)(m.total / row), row, row, m.Pb, row);
 }
 
 bool ensure_cap(Mlp &m, int B)
@@ -242,12 +256,12 @@ bool ensure_cap(Mlp &m, int B)
     const int h = m.hid, mx = std::max(m.hid, m.outp[kLayers - 1]);
     if (!m.alloc(&m.xs, (size_t)B * m.nin) || !m.alloc(&m.ts, (size_t)B * m.nout) ||
         !m.alloc(&m.dys, (size_t)B * m.nout) || !m.alloc(&m.X, (size_t)B * m.inp[0]) ||
-        !m.alloc(&m.XT, (size_t)m.inp[0] * B) || !m.alloc(&m.Y, (size_t)B * m.nout) ||
-        !m.alloc(&m.dZf, (size_t)B * mx) || !m.alloc(&m.dH, (size_t)B * h) || !m.alloc(&m.dX, (size_t)B * m.inp[0]) ||
-        !m.alloc(&m.dZb, (size_t)B * mx) || !m.alloc(&m.dZbT, (size_t)mx * B))
+        !m.alloc(&m.Y, (size_t)B * m.nout) || !m.alloc(&m.dX, (size_t)B * m.inp[0]))
         return false;
+    for (int p = 0; p < 2; p++)
+        if (!m.alloc(&m.dZf[p], (size_t)B * mx) || !m.alloc(&m.dZb[p], (size_t)B * mx)) return false;
     for (int l = 1; l < kLayers; l++)
-        if (!m.alloc(&m.H[l], (size_t)B * h) || !m.alloc(&m.HT[l], (size_t)h * B) || !m.alloc(&m.Z[l], (size_t)B * h))
+        if (!m.alloc(&m.H[l], (size_t)B * h) || !m.alloc(&m.Z[l], (size_t)B * h))
             return false;
     m.cap = B;
     return true;
@@ -263,8 +277,8 @@ GemmArgs gemm(const Mlp &m, const __nv_bfloat16 *A, int lda, const __nv_bfloat16
 
 bool forward(Mlp &m, int B)
 {
-    note_launch();
-    k_pack_bf16<<<blocks_for((long long)B * m.inp[0]), 256, 0, m.st>>>(m.xs, B, m.nin, m.nin, m.X, m.inp[0]);
+    if (!launch_chained(k_pack_bf16, blocks_for((long long)B * m.inp[0]), m.st, m.xs, B, m.nin, m.nin, m.X, m.inp[0]))
+        return false;
     const __nv_bfloat16 *hin = m.X;
     int ldin = m.inp[0];
     for (int l = 0; l < kLayers; l++) {
@@ -284,47 +298,35 @@ bool forward(Mlp &m, int B)
     return true;
 }
 
-// backward from dZ of the last layer (already in dZf / dZb); weight grads
-// when `weights`, dX when `input`
+// backward from dZ of the last layer (already in dZf[1] / dZb[1]); weight
+// grads when `weights`, dX when `input`.  Per layer one launch: dW = dZ^T H (both
+// operands read transposed), db, and dZ of the layer below (dH times GELU' in
+// the epilogue), which goes to the other buffer.
 bool backward(Mlp &m, int B, bool weights, bool input)
 {
     for (int l = kLayers - 1; l >= 0; l--) {
-        const int o = m.out[l], op = m.outp[l], ld = (l == kLayers - 1) ? op : m.hid;
-        if (weights) {
-            note_launch();
-            k_col_sum<<<(o + 127) / 128, 128, 0, m.st>>>(m.dZf, B, o, m.gb[l]);
-            note_launch();
-            k_transpose_bf16<<<blocks_for((long long)op * B), 256, 0, m.st>>>(m.dZb, B, o, ld, m.dZbT, op, B);
-            const __nv_bfloat16 *hT;
-            if (l == 0) {
-                note_launch();
-                k_transpose_bf16<<<blocks_for((long long)m.inp[0] * B), 256, 0, m.st>>>(m.X, B, m.inp[0], m.inp[0],
-                                                                                          m.XT, m.inp[0], B);
-                hT = m.XT;
-            } else {
-                note_launch();
-                k_transpose_bf16<<<blocks_for((long long)m.hid * B), 256, 0, m.st>>>(m.H[l], B, m.hid, m.hid, m.HT[l],
-                                                                                       m.hid, B);
-                hT = m.HT[l];
-            }
-            GemmArgs g = gemm(m, m.dZbT, B, hT, B, o, m.inp[l], B);
-            g.C32 = m.gW[l]; g.ldc32 = m.inp[l];
-            if (!gemm_bf16_launch(g, m.st)) return false;
-        }
+        const int o = m.out[l], op = m.outp[l], ld = (l == kLayers - 1) ? op : m.hid, p = l & 1;
+        GemmArgs dw = gemm(m, m.dZb[p], ld, l == 0 ? m.X : m.H[l], m.inp[l], o, m.inp[l], B);
+        dw.a_t = dw.b_t = true;
+        dw.C32 = m.gW[l]; dw.ldc32 = m.inp[l];
+        GemmArgs dh = gemm(m, m.dZb[p], ld, m.Wb[l], m.inp[l], B, m.inp[l], op);
+        dh.b_t = true;
         if (l > 0) {
-            GemmArgs g = gemm(m, m.dZb, ld, m.WbT[l], op, B, m.hid, op);
-            g.C32 = m.dH; g.ldc32 = m.hid;
-            if (!gemm_bf16_launch(g, m.st)) return false;
-            note_launch();
-            k_gelu_back<<<blocks_for((long long)B * m.hid), 256, 0, m.st>>>(m.dH, m.Z[l], (long long)B * m.hid,
-                                                                              m.dZf, m.dZb);
-        } else if (input) {
-            GemmArgs g = gemm(m, m.dZb, m.hid, m.WbT[0], m.hid, B, m.inp[0], m.hid);
-            g.C32 = m.dX; g.ldc32 = m.inp[0];
-            if (!gemm_bf16_launch(g, m.st)) return false;
+            dh.act = 2; dh.Zin = m.Z[l]; dh.ldz = m.hid;
+            dh.C32 = m.dZf[1 - p]; dh.ldc32 = m.hid;
+            dh.C16 = m.dZb[1 - p]; dh.ldc16 = m.hid;
+        } else {
+            dh.C32 = m.dX; dh.ldc32 = m.inp[0];
+        }
+        const bool down = l > 0 || input;
+        const ColSum cs{m.dZf[p], B, o, o, m.gb[l]};
+        if (weights) {
+            if (!gemm_bf16_group(dw, down ? &dh : nullptr, &cs, m.st)) return false;
+        } else if (down && !gemm_bf16_group(dh, nullptr, nullptr, m.st)) {
+            return false;
         }
     }
-    return cuda_ok(cudaGetLastError(), "mlp backward");
+    return true;
 }
 
 bool upload(Mlp &m, float *dst, const float *src, size_t count)
@@ -332,13 +334,16 @@ bool upload(Mlp &m, float *dst, const float *src, size_t count)
     return cuda_ok(cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyHostToDevice, m.st), "mlp H2D");
 }
 
-bool check_err(Mlp &m)
+// waits for the network's stream; the loss of the step when asked for
+bool check_err(Mlp &m, double *loss = nullptr)
 {
-    int e = 0;
-    if (!cuda_ok(cudaMemcpyAsync(&e, m.err, sizeof(int), cudaMemcpyDeviceToHost, m.st), "err D2H") ||
+    struct { double loss; int err, pad; } r{};
+    static_assert(sizeof r == 2 * sizeof(double), "status layout");
+    if (!cuda_ok(cudaMemcpyAsync(&r, m.loss, sizeof r, cudaMemcpyDeviceToHost, m.st), "status D2H") ||
         !cuda_ok(cudaStreamSynchronize(m.st), "mlp sync"))
         return false;
-    if (e) {
+    if (loss) *loss = r.loss;
+    if (r.err) {
         cudaMemsetAsync(m.err, 0, sizeof(int), m.st);
         set_error(FDTD_ERR_TIMEOUT, "surrogate: a tensor-core GEMM wait gave up");
         return false;
@@ -407,16 +412,10 @@ int fdtd_mlp_get_params(void *h, float *out)
     Mlp *m = net(h);
     if (!m || !out) return FDTD_ERR_ARG;
     if (!cuda_ok(cudaStreamSynchronize(m->st), "sync")) return fdtd_last_error();
-    size_t off = 0;
-    std::vector<float> w;
-    for (int l = 0; l < kLayers; l++) {
-        w.resize(m->wcount(l));
-        if (!cuda_ok(cudaMemcpy(w.data(), m->W[l], w.size() * 4, cudaMemcpyDeviceToHost), "D2H")) return fdtd_last_error();
-        for (int o = 0; o < m->out[l]; o++)
-            for (int i = 0; i < m->in[l]; i++) out[off++] = w[(size_t)o * m->inp[l] + i];
-        if (!cuda_ok(cudaMemcpy(out + off, m->b[l], m->out[l] * 4, cudaMemcpyDeviceToHost), "D2H")) return fdtd_last_error();
-        off += m->out[l];
-    }
+    std::vector<float> img((size_t)m->total);
+    if (!cuda_ok(cudaMemcpy(img.data(), m->P, img.size() * sizeof(float), cudaMemcpyDeviceToHost), "D2H"))
+        return fdtd_last_error();
+    m->flatten(img.data(), out);
     return FDTD_OK;
 }
 
@@ -426,19 +425,13 @@ int fdtd_mlp_set_params(void *h, const float *in)
     Mlp *m = net(h);
     if (!m || !in) return FDTD_ERR_ARG;
     if (!cuda_ok(cudaStreamSynchronize(m->st), "sync")) return fdtd_last_error();
-    size_t off = 0;
-    std::vector<float> w;
-    for (int l = 0; l < kLayers; l++) {
-        w.assign(m->wcount(l), 0.0f);
-        for (int o = 0; o < m->out[l]; o++)
-            for (int i = 0; i < m->in[l]; i++) w[(size_t)o * m->inp[l] + i] = in[off++];
-        if (!cuda_ok(cudaMemcpy(m->W[l], w.data(), w.size() * 4, cudaMemcpyHostToDevice), "H2D") ||
-            !cuda_ok(cudaMemcpy(m->b[l], in + off, m->out[l] * 4, cudaMemcpyHostToDevice), "H2D"))
-            return fdtd_last_error();
-        off += m->out[l];
-        cudaMemset(m->mW[l], 0, m->wcount(l) * 4); cudaMemset(m->vW[l], 0, m->wcount(l) * 4);
-        cudaMemset(m->mb[l], 0, m->out[l] * 4); cudaMemset(m->vb[l], 0, m->out[l] * 4);
-    }
+    std::vector<float> img((size_t)m->total);
+    m->unflatten(in, img.data());
+    const size_t bytes = img.size() * sizeof(float);
+    if (!cuda_ok(cudaMemcpyAsync(m->P, img.data(), bytes, cudaMemcpyHostToDevice, m->st), "H2D") ||
+        !cuda_ok(cudaMemsetAsync(m->Mo, 0, bytes, m->st), "memset") ||
+        !cuda_ok(cudaMemsetAsync(m->Vo, 0, bytes, m->st), "memset"))
+        return fdtd_last_error();
     m->step = 0;
     return refresh_bf16(*m) && check_err(*m) ? FDTD_OK : fdtd_last_error();
 }
@@ -454,19 +447,17 @@ int fdtd_mlp_forward(void *h, const float *x, int batch, float *y)
     return check_err(*m) ? FDTD_OK : fdtd_last_error();
 }
 
-static int grads_common(Mlp *m, const float *x, const float *t, int batch, double *loss)
+static int grads_common(Mlp *m, const float *x, const float *t, int batch)
 {
     if (!ensure_cap(*m, batch) || !upload(*m, m->xs, x, (size_t)batch * m->nin) ||
         !upload(*m, m->ts, t, (size_t)batch * m->nout) || !forward(*m, batch))
         return fdtd_last_error();
     if (!cuda_ok(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st), "memset")) return fdtd_last_error();
     const int L = kLayers - 1;
-    note_launch();
-    k_mse<<<blocks_for((long long)batch * m->outp[L]), 256, 0, m->st>>>(m->Y, m->ts, batch, m->nout, m->outp[L],
-                                                                          m->dZf, m->dZb, m->loss);
-    if (!backward(*m, batch, true, false)) return fdtd_last_error();
-    if (loss && !cuda_ok(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st), "D2H"))
+    if (!launch_chained(k_mse, blocks_for((long long)batch * m->outp[L]), m->st, m->Y, m->ts, batch, m->nout, m->outp[L],
+                        m->dZf[1], m->dZb[1], m->loss))
         return fdtd_last_error();
+    if (!backward(*m, batch, true, false)) return fdtd_last_error();
     return FDTD_OK;
 }
 
@@ -475,19 +466,13 @@ int fdtd_mlp_gradients(void *h, const float *x, const float *t, int batch, float
     std::lock_guard<std::mutex> lock(api_mutex());
     Mlp *m = net(h);
     if (!batch_ok(m, batch) || !x || !t) return FDTD_ERR_ARG;
-    int r = grads_common(m, x, t, batch, loss);
-    if (r != FDTD_OK || !check_err(*m)) return r != FDTD_OK ? r : fdtd_last_error();
+    int r = grads_common(m, x, t, batch);
+    if (r != FDTD_OK || !check_err(*m, loss)) return r != FDTD_OK ? r : fdtd_last_error();
     if (grad) {
-        size_t off = 0;
-        std::vector<float> w;
-        for (int l = 0; l < kLayers; l++) {
-            w.resize(m->wcount(l));
-            if (!cuda_ok(cudaMemcpy(w.data(), m->gW[l], w.size() * 4, cudaMemcpyDeviceToHost), "D2H")) return fdtd_last_error();
-            for (int o = 0; o < m->out[l]; o++)
-                for (int i = 0; i < m->in[l]; i++) grad[off++] = w[(size_t)o * m->inp[l] + i];
-            if (!cuda_ok(cudaMemcpy(grad + off, m->gb[l], m->out[l] * 4, cudaMemcpyDeviceToHost), "D2H")) return fdtd_last_error();
-            off += m->out[l];
-        }
+        std::vector<float> img((size_t)m->total);
+        if (!cuda_ok(cudaMemcpy(img.data(), m->G, img.size() * sizeof(float), cudaMemcpyDeviceToHost), "D2H"))
+            return fdtd_last_error();
+        m->flatten(img.data(), grad);
     }
     return FDTD_OK;
 }
@@ -497,20 +482,15 @@ int fdtd_mlp_train_step(void *h, const float *x, const float *t, int batch, floa
     std::lock_guard<std::mutex> lock(api_mutex());
     Mlp *m = net(h);
     if (!batch_ok(m, batch) || !x || !t || !(lr > 0)) return FDTD_ERR_ARG;
-    int r = grads_common(m, x, t, batch, loss);
+    int r = grads_common(m, x, t, batch);
     if (r != FDTD_OK) return r;
     m->step++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.0f - std::pow(b1, (float)m->step), c2 = 1.0f - std::pow(b2, (float)m->step);
-    for (int l = 0; l < kLayers; l++) {
-        note_launch(2);
-        k_adam<<<blocks_for(m->wcount(l)), 256, 0, m->st>>>(m->W[l], m->gW[l], m->mW[l], m->vW[l], m->wcount(l), lr, b1,
-                                                           b2, eps, c1, c2);
-        k_adam<<<blocks_for(m->out[l]), 256, 0, m->st>>>(m->b[l], m->gb[l], m->mb[l], m->vb[l], m->out[l], lr, b1, b2,
-                                                        eps, c1, c2);
-    }
-    if (!refresh_bf16(*m)) return fdtd_last_error();
-    return check_err(*m) ? FDTD_OK : fdtd_last_error();
+    if (!launch_chained(k_adam, blocks_for(m->total / 4), m->st, (float4 *)m->P, (const float4 *)m->G, (float4 *)m->Mo,
+                        (float4 *)m->Vo, (__nv_bfloat162 *)m->Pb, m->total / 4, lr, b1, b2, eps, c1, c2))
+        return fdtd_last_error();
+    return check_err(*m, loss) ? FDTD_OK : fdtd_last_error();
 }
 
 int fdtd_mlp_input_gradient(void *h, const float *x, const float *dy, int batch, float *dx)
@@ -522,9 +502,9 @@ int fdtd_mlp_input_gradient(void *h, const float *x, const float *dy, int batch,
         !upload(*m, m->dys, dy, (size_t)batch * m->nout) || !forward(*m, batch))
         return fdtd_last_error();
     const int L = kLayers - 1;
-    note_launch();
-    k_seed_grad<<<blocks_for((long long)batch * m->outp[L]), 256, 0, m->st>>>(m->dys, batch, m->nout, m->outp[L],
-                                                                                m->dZf, m->dZb);
+    if (!launch_chained(k_seed_grad, blocks_for((long long)batch * m->outp[L]), m->st, m->dys, batch, m->nout,
+                        m->outp[L], m->dZf[1], m->dZb[1]))
+        return fdtd_last_error();
     if (!backward(*m, batch, false, true)) return fdtd_last_error();
     std::vector<float> full((size_t)batch * m->inp[0]);
     if (!cuda_ok(cudaMemcpyAsync(full.data(), m->dX, full.size() * 4, cudaMemcpyDeviceToHost, m->st), "D2H") ||
