@@ -29,6 +29,7 @@
 // last row replaced by ones, right-hand side n e_n.  The reference stores the
 // last Arnoldi norm one element past its size x size matrix
 // (mode.c:3542-3544 with i = size); that value is never read and is not kept.
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -67,118 +68,369 @@ struct MsGeom {
     double disc, omega2;
     const double2 *ep, *mu, *pml;   // 3, 3, 2 per cell
     const double2 *inv_epz, *inv_muz; // 1 per cell
+    const double *inv_s2;             // 2 per cell: 1 / |sx|^2, 1 / |sy|^2
 };
 
-// per-cell 1/ep_z and 1/mu_z (complex_reciprocal)
-__global__ void k_ms_inverses(MsGeom g, double2 *inv_epz, double2 *inv_muz)
+// per-cell 1/ep_z and 1/mu_z (complex_reciprocal), and the real factor of a
+// division by sx or sy (cdiv), so that the operator divides by multiplying
+__global__ void k_ms_inverses(MsGeom g, double2 *inv_epz, double2 *inv_muz, double *inv_s2)
 {
     const int n = g.mi * g.mj;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         inv_epz[c] = crecip(g.ep[3 * c + 2]);
         inv_muz[c] = crecip(g.mu[3 * c + 2]);
+        for (int w = 0; w < 2; w++) {
+            const double m = cmag(g.pml[2 * c + w]);
+            inv_s2[2 * c + w] = __ddiv_rn(1.0, dmul(m, m));
+        }
     }
 }
 
-// out = B in on interior cells (mode.c:2796-2943), 0 on the window edge.
-// Vectors: v[2c] = Hx, v[2c+1] = Hy.
-__global__ void k_ms_beta2(MsGeom g, const double2 *__restrict__ in, double2 *__restrict__ out)
+// One component of (B in) at cell c (mode.c:2796-2943), w = 0 Hx, 1 Hy; 0 on
+// the window edge.  Vectors: v[2c] = Hx, v[2c+1] = Hy.  The two components'
+// formulas are each other's with x and y exchanged: n is the neighbour behind
+// (left for Hx, below for Hy), q the one ahead across (above, right).  Loads
+// go through L2: inside the Krylov kernel other blocks wrote `in`.
+__device__ __forceinline__ double2 ms_beta2(const MsGeom &g, const double2 *in, int c, int w)
 {
-    const int mi = g.mi, mj = g.mj, n = mi * mj;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const int i = c % mi, j = c / mi;
-        if (i < 1 || i > mi - 2 || j < 1 || j > mj - 2) {
-            out[2 * c] = make_double2(0.0, 0.0);
-            out[2 * c + 1] = make_double2(0.0, 0.0);
-            continue;
-        }
-        const double d = 1.0 / g.disc;
-        const int r = c + 1, l = c - 1, u = c + mi, dn = c - mi, dr = c - mi + 1, ul = c + mi - 1;
-        const double2 Hx = in[2 * c], Hx_r = in[2 * r], Hx_l = in[2 * l], Hx_u = in[2 * u], Hx_d = in[2 * dn],
-                      Hx_dr = in[2 * dr];
-        const double2 Hy = in[2 * c + 1], Hy_r = in[2 * r + 1], Hy_l = in[2 * l + 1], Hy_u = in[2 * u + 1],
-                      Hy_d = in[2 * dn + 1], Hy_ul = in[2 * ul + 1];
-        const double2 Bx = cmul(g.mu[3 * c], Hx), Bx_r = cmul(g.mu[3 * r], Hx_r), Bx_l = cmul(g.mu[3 * l], Hx_l),
-                      Bx_d = cmul(g.mu[3 * dn], Hx_d), Bx_dr = cmul(g.mu[3 * dr], Hx_dr);
-        const double2 By = cmul(g.mu[3 * c + 1], Hy), By_u = cmul(g.mu[3 * u + 1], Hy_u),
-                      By_d = cmul(g.mu[3 * dn + 1], Hy_d), By_l = cmul(g.mu[3 * l + 1], Hy_l),
-                      By_ul = cmul(g.mu[3 * ul + 1], Hy_ul);
-        const double2 imz = g.inv_muz[c], imz_l = g.inv_muz[l], imz_d = g.inv_muz[dn];
-        const double2 iez = g.inv_epz[c], iez_r = g.inv_epz[r], iez_u = g.inv_epz[u];
-        const double2 sx = g.pml[2 * c], sx_u = g.pml[2 * u], sx_d = g.pml[2 * dn], sx_r = g.pml[2 * r],
-                      sx_l = g.pml[2 * l];
-        const double2 sy = g.pml[2 * c + 1], sy_u = g.pml[2 * u + 1], sy_d = g.pml[2 * dn + 1],
-                      sy_r = g.pml[2 * r + 1], sy_l = g.pml[2 * l + 1];
-        (void)sx_d;
-        const double2 Bx_dx = cdiv(csmul(d, csub(Bx_r, Bx)), sx);
-        const double2 Bx_dx_l = cdiv(csmul(d, csub(Bx, Bx_l)), sx_l);
-        const double2 Bx_dx_d = cdiv(csmul(d, csub(Bx_dr, Bx_d)), sx_d);
-        const double2 By_dy = cdiv(csmul(d, csub(By_u, By)), sy);
-        const double2 By_dy_d = cdiv(csmul(d, csub(By, By_d)), sy_d);
-        const double2 By_dy_l = cdiv(csmul(d, csub(By_ul, By_l)), sy_l);
-        const double2 Hx_dy = cdiv(csmul(d, csub(Hx, Hx_d)), sy);
-        const double2 Hx_dy_u = cdiv(csmul(d, csub(Hx_u, Hx)), sy_u);
-        const double2 Hx_dy_r = cdiv(csmul(d, csub(Hx_r, Hx_dr)), sy_r);
-        const double2 Hy_dx = cdiv(csmul(d, csub(Hy, Hy_l)), sx);
-        const double2 Hy_dx_r = cdiv(csmul(d, csub(Hy_r, Hy)), sx_r);
-        const double2 Hy_dx_u = cdiv(csmul(d, csub(Hy_u, Hy_ul)), sx_u);
-        const double2 epx = g.ep[3 * c], epy = g.ep[3 * c + 1];
-        const double2 x1 = cdiv(csmul(d, csub(cmul(imz, Bx_dx), cmul(imz_l, Bx_dx_l))), sx);
-        const double2 x2 = cdiv(csmul(d, csub(cmul(imz, By_dy), cmul(imz_l, By_dy_l))), sx);
-        const double2 x3 = cdiv(cmul(csmul(-d, epy), csub(cmul(iez_u, Hy_dx_u), cmul(iez, Hy_dx))), sy);
-        const double2 x4 = cdiv(cmul(csmul(d, epy), csub(cmul(iez_u, Hx_dy_u), cmul(iez, Hx_dy))), sy);
-        const double2 x5 = csmul(g.omega2, cmul(cmul(epy, g.mu[3 * c]), Hx));
-        const double2 y1 = cdiv(csmul(d, csub(cmul(imz, Bx_dx), cmul(imz_d, Bx_dx_d))), sy);
-        const double2 y2 = cdiv(csmul(d, csub(cmul(imz, By_dy), cmul(imz_d, By_dy_d))), sy);
-        const double2 y3 = cdiv(cmul(csmul(d, epx), csub(cmul(iez_r, Hy_dx_r), cmul(iez, Hy_dx))), sx);
-        const double2 y4 = cdiv(cmul(csmul(-d, epx), csub(cmul(iez_r, Hx_dy_r), cmul(iez, Hx_dy))), sx);
-        const double2 y5 = csmul(g.omega2, cmul(cmul(epx, g.mu[3 * c + 1]), Hy));
-        out[2 * c] = cadd(cadd(cadd(x1, x2), cadd(x3, x4)), x5);
-        out[2 * c + 1] = cadd(cadd(cadd(y1, y2), cadd(y3, y4)), y5);
-    }
+    const int mi = g.mi, mj = g.mj;
+    const int i = c % mi, j = c / mi;
+    if (i < 1 || i > mi - 2 || j < 1 || j > mj - 2) return make_double2(0.0, 0.0);
+    const double d = __ddiv_rn(1.0, g.disc);
+    auto H = [&](int cell, int comp) { return __ldcg(in + 2 * cell + comp); };
+    auto B = [&](int cell, int comp) { return cmul(g.mu[3 * cell + comp], H(cell, comp)); };
+    // cdiv(x, s) of a stretch factor s: x conj(s) / |s|^2
+    auto over = [&](double2 x, int cell, int comp) {
+        return csmul(g.inv_s2[2 * cell + comp], cmul(x, cconj(g.pml[2 * cell + comp])));
+    };
+    auto dB = [&](int cell, int comp) {   // dBx/dx or dBy/dy at a cell (forward)
+        return over(csmul(d, csub(B(cell + (comp ? mi : 1), comp), B(cell, comp))), cell, comp);
+    };
+    auto dH = [&](int cell, int comp) {   // dHx/dy or dHy/dx at a cell (backward)
+        return over(csmul(d, csub(H(cell, comp), H(cell - (comp ? 1 : mi), comp))), cell, 1 - comp);
+    };
+    const int n = w ? c - mi : c - 1, q = w ? c + 1 : c + mi;
+    const double2 imz = g.inv_muz[c], imz_n = g.inv_muz[n], iez = g.inv_epz[c], iez_q = g.inv_epz[q];
+    const double2 e = g.ep[3 * c + 1 - w];
+    const double2 t1 = over(csmul(d, csub(cmul(imz, dB(c, 0)), cmul(imz_n, dB(n, 0)))), c, w);
+    const double2 t2 = over(csmul(d, csub(cmul(imz, dB(c, 1)), cmul(imz_n, dB(n, 1)))), c, w);
+    const double2 t3 = over(cmul(csmul(w ? d : -d, e), csub(cmul(iez_q, dH(q, 1)), cmul(iez, dH(c, 1)))), c, 1 - w);
+    const double2 t4 = over(cmul(csmul(w ? -d : d, e), csub(cmul(iez_q, dH(q, 0)), cmul(iez, dH(c, 0)))), c, 1 - w);
+    const double2 t5 = csmul(g.omega2, cmul(cmul(e, g.mu[3 * c + w]), H(c, w)));
+    return cadd(cadd(cadd(t1, t2), cadd(t3, t4)), t5);
+}
+
+__global__ void k_ms_beta2(MsGeom g, const double2 *in, double2 *out)
+{
+    const int n2 = 2 * g.mi * g.mj;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n2; t += gridDim.x * blockDim.x)
+        out[t] = ms_beta2(g, in, t >> 1, t & 1);
 }
 
 // ---- inner products: disc^2 * sum conj(a) b over (Hx, Hy) -----------------
-// Blocks write partials; the last block to finish (completion count after a
-// fence) adds them in block order and writes *out (optionally also
-// sqrt(|out|) to *norm_out) and resets the count.  Deterministic.
+// Element t belongs to thread t % (kDotBlocks kDotThreads) of the grid; threads,
+// warps and blocks add in a fixed order, whichever kernel does it, so every
+// inner product is deterministic.
 constexpr int kDotBlocks = 148, kDotThreads = 256;
+constexpr int kDotStride = kDotBlocks * kDotThreads;
 
+__device__ __forceinline__ void dot_add(double2 &s, double2 a, double2 b)
+{
+    s = cadd(s, cmul(cconj(a), b));
+}
+
+// sum over the warp in a fixed tree, the same bits in every lane
+__device__ __forceinline__ double2 dot_warp(double2 s, int width)
+{
+    for (int o = width / 2; o > 0; o >>= 1) {
+        s.x = dadd(s.x, __shfl_xor_sync(0xffffffffu, s.x, o));
+        s.y = dadd(s.y, __shfl_xor_sync(0xffffffffu, s.y, o));
+    }
+    return s;
+}
+
+// the block's sum, in every thread (ws: one value a warp)
+__device__ __forceinline__ double2 dot_block(double2 s, double2 *ws)
+{
+    s = dot_warp(s, 32);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+    __syncthreads();
+    return dot_warp(ws[threadIdx.x & (kDotThreads / 32 - 1)], kDotThreads / 32);
+}
+static_assert(kDotBlocks <= kDotThreads, "one thread a block's partial");
+
+// one inner product: the last block to finish (completion count after a fence)
+// adds the partials and writes *out (optionally also sqrt(|out|) to *norm_out)
 __global__ void __launch_bounds__(kDotThreads) k_ms_dot(const double2 *a, const double2 *b, int n2, double disc2,
                                                       double2 *partials, unsigned *done, double2 *out,
                                                       double *norm_out)
 {
-    double sre = 0.0, sim = 0.0;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n2; t += gridDim.x * blockDim.x) {
-        const double2 p = cmul(cconj(a[t]), b[t]);
-        sre = dadd(sre, p.x);
-        sim = dadd(sim, p.y);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        sre = dadd(sre, __shfl_down_sync(0xffffffffu, sre, o));
-        sim = dadd(sim, __shfl_down_sync(0xffffffffu, sim, o));
-    }
-    __shared__ double2 ws[kDotThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) ws[warp] = make_double2(sre, sim);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 v = ws[0];
-        for (int w = 1; w < kDotThreads / 32; w++) v = cadd(v, ws[w]);
-        partials[blockIdx.x] = v;
-    }
+    __shared__ double2 ws[2][kDotThreads / 32];
     __shared__ bool last;
-    __threadfence();
+    double2 s = make_double2(0.0, 0.0);
+    for (int t = blockIdx.x * kDotThreads + threadIdx.x; t < n2; t += kDotStride) dot_add(s, a[t], b[t]);
+    s = dot_block(s, ws[0]);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last || threadIdx.x != 0) return;
+    if (!last) return;
     __threadfence();
-    double2 s = partials[0];
-    for (int p = 1; p < (int)gridDim.x; p++) s = cadd(s, partials[p]);
-    s = csmul(disc2, s);
-    *out = s;
-    if (norm_out) *norm_out = __dsqrt_rn(cmag(s));
-    *done = 0u;
+    // every partial fetched at once (one thread walking them took 9 of a dot's 11 us)
+    s = threadIdx.x < gridDim.x ? __ldcg(partials + threadIdx.x) : make_double2(0.0, 0.0);
+    s = csmul(disc2, dot_block(s, ws[1]));
+    if (threadIdx.x == 0) {
+        *out = s;
+        if (norm_out) *norm_out = __dsqrt_rn(cmag(s));
+        *done = 0u;
+    }
+}
+
+// ---- one Krylov cycle in one cooperative launch ----------------------------
+// k_i = B k_{i-1} for i = 1..K with modified Gram-Schmidt,
+//   h_j = <k_j, y - sum_{l<j} h_l k_l>,  y = B k_{i-1}.
+//
+// What bounds it: as kernels a cycle was 470 launches of 2 to 11 us, each
+// waiting for the one before (K = 20, 200 x 160 window: 4.3 ms a cycle, the
+// arithmetic a few percent of it).  In one launch, with y in registers and the
+// basis in L2, each of the K (K + 1) / 2 + K inner products still costs a
+// round trip of the grid through L2, 2 x 1.4 us between the two dies: 0.95 ms a
+// cycle.  So the products of a step are taken together (low-synchronisation
+// Gram-Schmidt, Swirydowicz, Langou, Ananthan, Yang, Thomas, 2021): with
+// s_j = <k_j, y> and the Gram matrix G_jl = <k_j, k_l>, whose row i - 1 rides
+// along in the same pass, the h above solve (I + strict lower triangle of G)
+// h = s, the same numbers to rounding.  A step is then two reductions (h,
+// norm) and a barrier: 0.35 ms a cycle, of which 0.15 are its 100 hops.
+//
+// Reductions: a block's partial sums, one word pair a value, go to the block
+// that adds that value up, and the sums to every block.  A word is 16 bytes, a
+// double and the reduction's number, written and read whole; the reader polls
+// the words themselves, so a hop is one write and one read and needs no fence.
+// (A counting barrier and reading the partials after it took as long as both
+// hops; every block reading every partial sent 44,000 reads to 37 cache
+// lines, slower than the second hop.)  Words are reused by the next reduction:
+// a block writes its partials only after it read every sum of this one, and
+// the sums were written after every partial was read.
+//
+// EPT elements of y a thread stay in registers; EPT = 0 keeps y in memory, for
+// windows over 75,000 cells.  The blocks are co-resident (cooperative
+// launch).  A wait longer than wait_ns sets *err; every later wait sees it and
+// the launch ends.
+struct MsKrylov {
+    MsGeom g;
+    double2 *basis;      // K + 1 vectors; k_0 given
+    int K, confinement;
+    double disc2;
+    double2 *H;          // K x K row-major: column i - 1 of step i
+    double *norm;        // norm[i] = |k_i|
+    ulonglong2 *words;   // partials [value][block](re, im), then sums [value] kWordStride apart; zero at launch
+    unsigned *bar;       // zero at launch
+    int *err;
+    double2 *gram;       // K x K for each block, when it does not fit shared memory
+    unsigned long long wait_ns;
+};
+constexpr int kWordStride = 8;   // a sum's words on a cache line of their own: every block polls them
+
+__device__ __forceinline__ unsigned long long ms_clock()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// polls done() until it holds; false when the wait gave up (here or elsewhere)
+template <typename F> __device__ __forceinline__ bool ms_poll(const MsKrylov &a, F done)
+{
+    unsigned long long t0 = 0;
+    for (unsigned tries = 1; !done(); tries++) {
+        if (tries % 64) continue;
+        if (*(volatile int *)a.err) return false;
+        const unsigned long long now = ms_clock();
+        if (!t0) t0 = now;
+        else if (now - t0 > a.wait_ns) {
+            atomicExch(a.err, 1);
+            return false;
+        }
+    }
+    return true;
+}
+
+// grid barrier k (1, 2, ...), by one thread of each block
+__device__ __forceinline__ bool ms_barrier(const MsKrylov &a, unsigned k)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    const unsigned target = k * gridDim.x;
+    return ms_poll(a, [&]() {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+        return v >= target;
+    });
+}
+
+// a 16-byte word (value, number of its inner product), written and read whole
+__device__ __forceinline__ void ms_publish(ulonglong2 *w, double v, unsigned long long n)
+{
+    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(w),
+                 "l"((unsigned long long)__double_as_longlong(v)), "l"(n)
+                 : "memory");
+}
+__device__ __forceinline__ bool ms_read(const ulonglong2 *w, unsigned long long n, double &v)
+{
+    unsigned long long lo, hi;
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(w)
+                 : "memory");
+    v = __longlong_as_double((long long)lo);
+    return hi == n;
+}
+
+// the sum of s over the warp to w[0] (every lane calls it)
+__device__ __forceinline__ void warp_sum_to(double2 *w, double2 s)
+{
+    s = dot_warp(s, 32);
+    if ((threadIdx.x & 31) == 0) *w = s;
+}
+
+constexpr int kDotWarps = kDotThreads / 32;
+__host__ __device__ constexpr size_t ms_shared(int K, bool gram)
+{
+    return ((size_t)(kDotWarps + 1) * 2 * K + (gram ? (size_t)K * K : 0)) * sizeof(double2);
+}
+
+template <int EPT> __global__ void __launch_bounds__(kDotThreads) k_ms_krylov(MsKrylov a)
+{
+    extern __shared__ __align__(16) double2 dyn[];
+    __shared__ double2 ws[2][kDotWarps];
+    __shared__ int ok;
+    const int n2 = 2 * a.g.mi * a.g.mj, tid = threadIdx.x, nb = gridDim.x, K = a.K;
+    const int warp = tid >> 5, lane = tid & 31;
+    const int t0 = blockIdx.x * kDotThreads + tid;
+    constexpr int R = EPT > 0 ? EPT : 1;
+    double2 *wsum = dyn;                         // [warp][2K]: the warps' sums of a reduction
+    double2 *sums = dyn + kDotWarps * 2 * K;     // [2K]: its result
+    double2 *G = a.gram ? a.gram + (size_t)blockIdx.x * K * K : sums + 2 * K;
+    ulonglong2 *part = a.words, *total = a.words + (size_t)4 * K * kDotBlocks;
+    double2 yr[R], qr[R];       // y and k_{i-1}
+    unsigned nbar = 0, nred = 0;
+    double2 *ym = nullptr;      // EPT = 0: y in memory
+    // f(element, slot, its value) for this thread's elements, in order
+    auto each = [&](auto f) {
+        if constexpr (EPT > 0) {
+#pragma unroll
+            for (int e = 0; e < R; e++)
+                if (t0 + e * kDotStride < n2) f(t0 + e * kDotStride, e, yr[e]);
+        } else {
+            for (int t = t0; t < n2; t += kDotStride) f(t, 0, ym[t]);
+        }
+    };
+    // sums[0..m) = the grid's sums of wsum[.][0..m); false when a wait gave up
+    auto reduce = [&](int m) -> bool {
+        nred++;
+        __syncthreads();
+        for (int v = tid; v < m; v += kDotThreads) {
+            double2 s = wsum[v];
+            for (int w = 1; w < kDotWarps; w++) s = cadd(s, wsum[w * 2 * K + v]);
+            ulonglong2 *p = part + 2 * ((size_t)v * kDotBlocks + blockIdx.x);
+            ms_publish(p, s.x, nred);
+            ms_publish(p + 1, s.y, nred);
+        }
+        bool good = true;
+        for (int v = blockIdx.x, q = 0; v < m; v += nb, q ^= 1) {   // values this block adds up
+            double2 s = make_double2(0.0, 0.0);
+            if (tid < nb) {
+                const ulonglong2 *p = part + 2 * ((size_t)v * kDotBlocks + tid);
+                good = ms_poll(a, [&]() {
+                    const bool re = ms_read(p, nred, s.x), im = ms_read(p + 1, nred, s.y);
+                    return re && im;
+                }) && good;
+            }
+            s = csmul(a.disc2, dot_block(s, ws[q]));
+            if (tid < 2) ms_publish(total + v * kWordStride + tid, tid ? s.y : s.x, nred);
+        }
+        for (int u = tid; u < 2 * m && good; u += kDotThreads) {
+            double x = 0.0;
+            good = ms_poll(a, [&]() { return ms_read(total + (u >> 1) * kWordStride + (u & 1), nred, x); });
+            reinterpret_cast<double *>(sums)[u] = x;
+        }
+        return !__syncthreads_or(!good);
+    };
+    for (int i = 1; i <= K; i++) {
+        const double2 *prev = a.basis + (size_t)(i - 1) * n2;
+        ym = a.basis + (size_t)i * n2;
+        each([&](int t, int e, double2 &y) {
+            int c = t >> 1;
+            if (a.confinement == 1) {   // columns 0 and mi-1 copy their neighbours
+                const int x = c % a.g.mi;
+                c += x == 0 ? 1 : (x == a.g.mi - 1 ? -1 : 0);
+            }
+            y = ms_beta2(a.g, prev, c, t & 1);
+            if (EPT > 0) qr[e] = prev[t];
+        });
+        // s_l = <k_l, y> and row i - 1 of G, every l < i in one pass
+#pragma unroll 4
+        for (int l = 0; l < i; l++) {
+            const double2 *q = a.basis + (size_t)l * n2;
+            double2 s = make_double2(0.0, 0.0), gs = s;
+            each([&](int t, int e, double2 &y) {
+                const double2 x = q[t];
+                dot_add(s, x, y);
+                dot_add(gs, EPT > 0 ? qr[e] : prev[t], x);
+            });
+            warp_sum_to(wsum + warp * 2 * K + l, s);
+            if (l + 1 < i) warp_sum_to(wsum + warp * 2 * K + i + l, gs);
+        }
+        if (!reduce(2 * i - 1)) return;
+        for (int l = tid; l + 1 < i; l += kDotThreads) G[(size_t)(i - 1) * K + l] = sums[i + l];
+        __syncthreads();
+        // h from (I + strictly lower G) h = s, in place, by one warp
+        if (warp == 0) {
+            if (K <= 32) {
+                double2 h = lane < i ? sums[lane] : make_double2(0.0, 0.0);
+                for (int j = 0; j + 1 < i; j++) {
+                    const double2 hj = make_double2(__shfl_sync(0xffffffffu, h.x, j), __shfl_sync(0xffffffffu, h.y, j));
+                    if (lane > j && lane < i) h = csub(h, cmul(hj, G[(size_t)lane * K + j]));
+                }
+                if (lane < i) sums[lane] = h;
+            } else {
+                for (int j = 0; j + 1 < i; j++) {
+                    const double2 hj = sums[j];
+                    for (int k = j + 1 + lane; k < i; k += 32) sums[k] = csub(sums[k], cmul(hj, G[(size_t)k * K + j]));
+                    __syncwarp();
+                }
+            }
+        }
+        __syncthreads();
+        if (blockIdx.x == 0)
+            for (int j = tid; j < i; j += kDotThreads) a.H[(size_t)j * K + (i - 1)] = sums[j];
+        if (i == K) break;
+#pragma unroll 4
+        for (int l = 0; l < i; l++) {
+            const double2 h = sums[l], *q = a.basis + (size_t)l * n2;
+            each([&](int t, int, double2 &y) { y = csub(y, cmul(h, q[t])); });
+        }
+        double2 s = make_double2(0.0, 0.0);
+        each([&](int, int, double2 &y) { dot_add(s, y, y); });
+        warp_sum_to(wsum + warp * 2 * K, s);
+        if (!reduce(1)) return;
+        const double norm = __dsqrt_rn(cmag(sums[0]));
+        if (t0 == 0) a.norm[i] = norm;
+        const double inv = __ddiv_rn(1.0, norm);
+        each([&](int t, int, double2 &y) {
+            y = csmul(inv, y);
+            if (EPT > 0) a.basis[(size_t)i * n2 + t] = y;
+        });
+        // the next application reads its neighbours' elements
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            ok = ms_barrier(a, ++nbar);
+        }
+        __syncthreads();
+        if (!ok) return;
+    }
 }
 
 // y -= (*coef) x
@@ -499,17 +751,19 @@ cd reference_sqrt(cd x)
     return cd(mag * re, mag * im);
 }
 
-struct DevBuf {
-    void *p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
+// one allocation handed out in 256-byte aligned pieces
+struct Slab {
+    char *p = nullptr;
+    size_t used = 0;
+    ~Slab() { if (p) cudaFree(p); }
+    template <typename T> size_t add(size_t count)
+    {
+        const size_t at = used;
+        used = (used + count * sizeof(T) + 255) / 256 * 256;
+        return at;
+    }
+    template <typename T> void at(size_t off, T **out) const { *out = (T *)(p + off); }
 };
-
-template <typename T> bool dev_alloc(DevBuf &b, size_t count, T **out)
-{
-    if (!cuda_ok(cudaMalloc(&b.p, count * sizeof(T) + 16), "cudaMalloc(mode solver)")) return false;
-    *out = (T *)b.p;
-    return true;
-}
 
 #define MSK(call)                                      \
     do {                                               \
@@ -520,12 +774,14 @@ struct Solver {
     int mi = 0, mj = 0, n = 0, n2 = 0;
     double disc = 0, omega = 0;
     cudaStream_t st = nullptr;
-    DevBuf b_ep, b_mu, b_pml, b_iez, b_imz, b_psi, b_basis, b_tmp, b_part, b_done, b_scal, b_norm, b_y, b_prev, b_f;
+    Slab slab;
     double2 *ep = nullptr, *mu = nullptr, *pml = nullptr, *iez = nullptr, *imz = nullptr;
     double2 *psi = nullptr, *basis = nullptr, *tmp = nullptr, *part = nullptr, *scal = nullptr, *y = nullptr;
-    double2 *prev = nullptr, *f = nullptr;
-    double *norm = nullptr;
-    unsigned *done = nullptr;
+    double2 *prev = nullptr, *f = nullptr, *gram = nullptr;
+    double *norm = nullptr, *is2 = nullptr;
+    unsigned *done = nullptr, *bar = nullptr;
+    ulonglong2 *words = nullptr;            // then bar, cleared together
+    int *err = nullptr;
     MsGeom g{};
 
     ~Solver()
@@ -536,28 +792,47 @@ struct Solver {
         }
     }
 
+    // partial and sum words of a cycle of K steps (2K values), then the barrier's count
+    static size_t words_count(size_t K) { return 2 * K * (2 * kDotBlocks + kWordStride) + 1; }
+    // the Gram matrix fits a block's shared memory
+    static bool gram_shared(size_t K) { return ms_shared((int)K, true) <= 200 * 1024; }
+
     bool setup(const mode &m, double om, int basis_vectors, int nprev)
     {
         mi = m.i; mj = m.j; n = mi * mj; n2 = 2 * n;
         disc = m.disc; omega = om;
         MSK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        if (!dev_alloc(b_ep, 3 * (size_t)n, &ep) || !dev_alloc(b_mu, 3 * (size_t)n, &mu) ||
-            !dev_alloc(b_pml, 2 * (size_t)n, &pml) || !dev_alloc(b_iez, n, &iez) || !dev_alloc(b_imz, n, &imz) ||
-            !dev_alloc(b_psi, n2, &psi) || !dev_alloc(b_basis, (size_t)basis_vectors * n2, &basis) ||
-            !dev_alloc(b_tmp, n2, &tmp) || !dev_alloc(b_part, kDotBlocks, &part) ||
-            !dev_alloc(b_done, 1, &done) || !dev_alloc(b_scal, (size_t)(basis_vectors + 1) * (basis_vectors + 1) + 8, &scal) ||
-            !dev_alloc(b_norm, (size_t)basis_vectors + 8, &norm) || !dev_alloc(b_y, basis_vectors + 1, &y) ||
-            !dev_alloc(b_prev, (size_t)(nprev > 0 ? nprev : 1) * n2, &prev) || !dev_alloc(b_f, 6 * (size_t)n, &f))
-            return false;
-        MSK(cudaMemsetAsync(done, 0, sizeof(unsigned), st));
+        const size_t nn = (size_t)n, kv = (size_t)basis_vectors, np = (size_t)(nprev > 0 ? nprev : 1);
+        const size_t o_ep = slab.add<double2>(3 * nn), o_mu = slab.add<double2>(3 * nn), o_pml = slab.add<double2>(2 * nn),
+                     o_iez = slab.add<double2>(nn), o_imz = slab.add<double2>(nn), o_is2 = slab.add<double>(2 * nn),
+                     o_psi = slab.add<double2>(2 * nn), o_basis = slab.add<double2>(kv * 2 * nn),
+                     o_tmp = slab.add<double2>(2 * nn), o_part = slab.add<double2>(kDotBlocks),
+                     o_words = slab.add<ulonglong2>(words_count(kv - 1)),
+                     o_done = slab.add<unsigned>(4), o_scal = slab.add<double2>((kv + 1) * (kv + 1) + 8),
+                     o_y = slab.add<double2>(kv + 1), o_prev = slab.add<double2>(np * 2 * nn),
+                     o_f = slab.add<double2>(6 * nn),
+                     o_gram = slab.add<double2>(gram_shared(kv - 1) ? 0 : kDotBlocks * (kv - 1) * (kv - 1));
+        MSK(cudaMalloc(&slab.p, slab.used));
+        slab.at(o_ep, &ep); slab.at(o_mu, &mu); slab.at(o_pml, &pml); slab.at(o_iez, &iez); slab.at(o_imz, &imz);
+        slab.at(o_is2, &is2); slab.at(o_psi, &psi); slab.at(o_basis, &basis); slab.at(o_tmp, &tmp);
+        slab.at(o_part, &part); slab.at(o_done, &done); slab.at(o_scal, &scal); slab.at(o_y, &y);
+        slab.at(o_prev, &prev); slab.at(o_f, &f);
+        slab.at(o_words, &words);
+        if (!gram_shared(kv - 1)) slab.at(o_gram, &gram);
+        bar = (unsigned *)(words + words_count(kv - 1) - 1);
+        err = (int *)(done + 2);
+        // after the K x K matrix H(r, c) = scal[1 + r K + c]: the norms, read back with it
+        norm = (double *)(scal + 1 + (kv - 1) * (kv - 1));
+        MSK(cudaMemsetAsync(done, 0, 4 * sizeof(unsigned), st));
+        MSK(cudaMemsetAsync(scal, 0, ((kv + 1) * (kv + 1) + 8) * sizeof(double2), st));
         static_assert(sizeof(complex) == sizeof(double2), "complex layout");
         MSK(cudaMemcpyAsync(ep, m.ep.m, 3 * (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, st));
         MSK(cudaMemcpyAsync(mu, m.mu.m, 3 * (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, st));
         MSK(cudaMemcpyAsync(pml, m.pml.m, 2 * (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, st));
         g.mi = mi; g.mj = mj; g.disc = disc; g.omega2 = om * om;
-        g.ep = ep; g.mu = mu; g.pml = pml; g.inv_epz = iez; g.inv_muz = imz;
+        g.ep = ep; g.mu = mu; g.pml = pml; g.inv_epz = iez; g.inv_muz = imz; g.inv_s2 = is2;
         note_launch();
-        k_ms_inverses<<<grid_blocks(n), 256, 0, st>>>(g, iez, imz);
+        k_ms_inverses<<<grid_blocks(n), 256, 0, st>>>(g, iez, imz, is2);
         return cuda_ok(cudaGetLastError(), "mode solver setup");
     }
 
@@ -597,7 +872,24 @@ struct Solver {
     void apply(const double2 *in, double2 *out)
     {
         note_launch();
-        k_ms_beta2<<<grid_blocks(n), 256, 0, st>>>(g, in, out);
+        k_ms_beta2<<<grid_blocks(n2), 256, 0, st>>>(g, in, out);
+    }
+    // k_1..k_K, H and the norms from k_0 (see k_ms_krylov)
+    bool krylov(int K, int confinement)
+    {
+        MsKrylov a{g, basis, K, confinement, disc * disc, scal + 1, norm, words, bar, err, gram, 1000000000ull};
+        MSK(cudaMemsetAsync(words, 0, words_count(K) * sizeof(ulonglong2), st));
+        const int per = (n2 + kDotStride - 1) / kDotStride;
+        const void *fn = per <= 1 ? (const void *)k_ms_krylov<1> : per <= 2 ? (const void *)k_ms_krylov<2>
+                         : per <= 4 ? (const void *)k_ms_krylov<4> : (const void *)k_ms_krylov<0>;
+        // blocks past the last element would only add zero partials
+        const int blocks = std::min(kDotBlocks, (n2 + kDotThreads - 1) / kDotThreads);
+        const size_t smem = ms_shared(K, !gram);
+        MSK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        void *args[] = {&a};
+        note_launch();
+        return cuda_ok(cudaLaunchCooperativeKernel(fn, dim3((unsigned)blocks), dim3(kDotThreads), args, smem, st),
+                       "Krylov cycle");
     }
 };
 
@@ -684,28 +976,19 @@ bool mode_solve_device(mode *psi, double omega, double tol, const mode *prev, in
         MSK(cudaMemcpyAsync(k0, s.psi, (size_t)n2 * sizeof(double2), cudaMemcpyDeviceToDevice, s.st));
         s.normalize(k0);
         s.bc(k0, confinement);
-        MSK(cudaMemsetAsync(Hd, 0, (size_t)K * K * sizeof(double2), s.st));
-        for (int i = 1; i <= K; i++) {
-            double2 *ki = s.basis + (size_t)i * n2;
-            s.apply(s.basis + (size_t)(i - 1) * n2, ki);
-            s.bc(ki, confinement);
-            for (int j = 0; j < i; j++) {
-                double2 *hji = Hd + (size_t)j * K + (i - 1);
-                s.dot(s.basis + (size_t)j * n2, ki, hji, nullptr);
-                s.axpy(ki, s.basis + (size_t)j * n2, hji);
-            }
-            if (i < K) {
-                // subdiagonal H(i, i-1) = |k_i|, then normalise
-                s.dot(ki, ki, s.scal, s.norm + i);
-                note_launch();
-                k_ms_scale<<<grid_blocks(n2), 256, 0, s.st>>>(ki, s.norm + i, n2);
-            }
-        }
-        MSK(cudaGetLastError());
-        std::vector<double> sub((size_t)K + 8);
-        MSK(cudaMemcpyAsync(Hh.data(), Hd, Hh.size() * sizeof(double2), cudaMemcpyDeviceToHost, s.st));
-        MSK(cudaMemcpyAsync(sub.data(), s.norm, (size_t)K * sizeof(double), cudaMemcpyDeviceToHost, s.st));
+        if (!s.krylov(K, confinement)) return false;
+        // H and, right after it, the norms
+        std::vector<double2> back((size_t)K * K + (K + 1) / 2);
+        MSK(cudaMemcpyAsync(back.data(), Hd, back.size() * sizeof(double2), cudaMemcpyDeviceToHost, s.st));
+        int late = 0;
+        MSK(cudaMemcpyAsync(&late, s.err, sizeof(int), cudaMemcpyDeviceToHost, s.st));
         MSK(cudaStreamSynchronize(s.st));
+        if (late) {
+            set_error(FDTD_ERR_TIMEOUT, "mode solver: a device-side wait gave up");
+            return false;
+        }
+        std::copy(back.begin(), back.begin() + (size_t)K * K, Hh.begin());
+        const double *sub = (const double *)(back.data() + (size_t)K * K);
         for (int r = 0; r < K; r++)
             for (int c = 0; c < K; c++) H[(size_t)r * K + c] = cd(Hh[(size_t)r * K + c].x, Hh[(size_t)r * K + c].y);
         for (int i = 1; i < K; i++) H[(size_t)i * K + (i - 1)] = cd(sub[i], 0.0);
@@ -736,8 +1019,7 @@ bool mode_solve_device(mode *psi, double omega, double tol, const mode *prev, in
         MSK(cudaMemcpyAsync(s.y, yd.data(), yd.size() * sizeof(double2), cudaMemcpyHostToDevice, s.st));
         note_launch();
         k_ms_combine<<<grid_blocks(n2), 256, 0, s.st>>>(s.psi, s.basis, s.y, K, n2);
-        MSK(cudaGetLastError());
-        MSK(cudaStreamSynchronize(s.st));   // yd is a host temporary
+        MSK(cudaGetLastError());   // yd is pageable: staged when the copy returned
         beta = reference_sqrt(lam);
         const cd n_eff = beta / omega;
         const double n_old = n_mag;
