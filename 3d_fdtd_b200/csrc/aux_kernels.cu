@@ -58,6 +58,36 @@ __global__ void k_overlap_finalize(const OverlapJob *jobs, int njobs, const doub
     overlap_finalize_job(jb, partials + (long long)jid * nparts, nparts, scale, dt, *step + step_offset);
 }
 
+// timefield3d_mode_overlap: one job, its argument, the partials and the sum in one
+// launch whose last block writes the value to pinned host memory.  The call is
+// latency: it was a job copy, two kernels and a copy back (9 us on the device),
+// now one kernel of 3 to 5.
+template <typename T>
+__global__ void __launch_bounds__(256) k_overlap_now(const T *const *f, int nx, int ny, OverlapJob jb, double2 *partials,
+                                                     unsigned *done, double scale, double2 *out)
+{
+    overlap_block<T>(f, nx, ny, jb, blockIdx.x, gridDim.x, partials + blockIdx.x);
+    __shared__ bool last;
+    __shared__ double2 stage[64];
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < gridDim.x) stage[threadIdx.x] = __ldcg(partials + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double sre = 0.0, sim = 0.0;
+    for (int p = 0; p < (int)gridDim.x; p++) {   // in order, as k_overlap_finalize
+        sre = dadd(sre, stage[p].x);
+        sim = dadd(sim, stage[p].y);
+    }
+    *out = make_double2(dmul(scale, sre), dmul(scale, sim));
+    *done = 0u;
+}
+
 // ---------------------------------------------------------------------------
 // End of one step of a run, in one launch: blocks [0, njobs*nparts) compute
 // the overlap partials of the fields just updated, the next `src_blocks`
@@ -345,6 +375,15 @@ int overlap_parts(long long cells)
 }
 
 template <typename T>
+void launch_overlap_now(const T *const *f_dev, int nx, int ny, const OverlapJob &job, double2 *partials, unsigned *done,
+                        double scale, double2 *out, cudaStream_t st)
+{
+    note_launch();
+    const int parts = overlap_parts((long long)job.win.wni * job.win.wnj);   // at most 64
+    k_overlap_now<T><<<parts, 256, 0, st>>>(f_dev, nx, ny, job, partials, done, scale, out);
+}
+
+template <typename T>
 void launch_overlap(const T *const *f_dev, int nx, int ny, const OverlapJob *jobs_dev, int njobs, long long cells,
                     double2 *partials, double scale, double dt, const long long *step, int step_offset,
                     cudaStream_t st)
@@ -414,6 +453,8 @@ void launch_check_finite(const float *a, long long n, int *bad, cudaStream_t st)
 }
 
 #define FDTD_INST(T)                                                                                               \
+    template void launch_overlap_now<T>(const T *const *, int, int, const OverlapJob &, double2 *, unsigned *,     \
+                                        double, double2 *, cudaStream_t);                                          \
     template void launch_overlap<T>(const T *const *, int, int, const OverlapJob *, int, long long, double2 *,     \
                                     double, double, const long long *, int, cudaStream_t);                         \
     template void launch_dft<T>(const T *const *, int, int, int, int, int, int, double, double, double2 *,         \

@@ -43,8 +43,8 @@ template <typename T> bool launch_explicit_or_zsection(Grid *g, double dt, int e
     CpmlView<T> c = cpml_view<T>(g, g->cur);
     SourcePlanes s = source_table(g);
     const bool cpml = !expl && g->boundary == FDTD_BOUNDARY_CPML;
-    if (efield) launch_update_E<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_e, cpml, expl, g->st);
-    else launch_update_H<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_m, true, cpml, expl, g->st);
+    if (efield) launch_update_E<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_e, cpml, expl, false, g->st);
+    else launch_update_H<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_m, true, cpml, expl, false, (T)g->dx, g->st);
     return cuda_ok(cudaGetLastError(), "interior update");
 }
 
@@ -595,23 +595,19 @@ complex timefield3d_mode_overlap(timefield3d psi, int center_x, int center_y, in
     j.reverse = reverse == 1;
     j.ratio = psi.disc / overlap_mode.disc;
     j.mode = dm->d;
-    j.inst = g->d_inst;
+    j.inst = nullptr;
     j.acc = nullptr;
     j.omega = nullptr;
     j.nfreq = 0;
     j.win = mode_window(g->nx, g->ny, j.cx, j.cy, j.mi, j.mj, j.ratio);
-    if (!cuda_ok(cudaMemcpyAsync(g->d_job1, &j, sizeof j, cudaMemcpyHostToDevice, g->st), "overlap job")) return inst;
     const double scale = (-0.5 * psi.disc * psi.disc);
-    const long long cells = (long long)j.win.wni * j.win.wnj;
     if (g->prec == FDTD_F64)
-        launch_overlap<double>((const double *const *)fptr(g), g->nx, g->ny, g->d_job1, 1, cells, g->d_partials, scale,
-                               0, g->d_step, 0, g->st);
+        launch_overlap_now<double>((const double *const *)fptr(g), g->nx, g->ny, j, g->d_partials, g->d_done, scale,
+                                   g->h_inst, g->st);
     else
-        launch_overlap<float>((const float *const *)fptr(g), g->nx, g->ny, g->d_job1, 1, cells, g->d_partials, scale,
-                              0, g->d_step, 0, g->st);
-    if (!cuda_ok(cudaMemcpyAsync(g->h_inst, g->d_inst, sizeof(double2), cudaMemcpyDeviceToHost, g->st), "overlap D2H") ||
-        !cuda_ok(cudaStreamSynchronize(g->st), "overlap sync"))
-        return inst;
+        launch_overlap_now<float>((const float *const *)fptr(g), g->nx, g->ny, j, g->d_partials, g->d_done, scale,
+                                  g->h_inst, g->st);
+    if (!cuda_ok(cudaGetLastError(), "overlap") || !cuda_ok(cudaStreamSynchronize(g->st), "overlap sync")) return inst;
     inst.re = g->h_inst->x;
     inst.im = g->h_inst->y;
     // cumulative += e^{i reduced phase} * inst, as timefield3d.c:3234-3236
@@ -960,6 +956,7 @@ int timefield3d_add_probe(timefield3d psi, int i, int j, int k, int m, int capac
     r.job.m = m;
     r.cap = capacity;
     g->probes.push_back(r);
+    if (i < 1 || i > psi.i - 2 || j < 1 || j > psi.j - 2 || k < 1 || k > psi.k - 2) g->probes_interior = false;
     int cap = 0;
     for (auto &p : g->probes) cap = std::max(cap, p.cap);
     cudaFree(g->d_probes); cudaFree(g->d_probe_buf); cudaFree(g->d_probe_count);
@@ -1004,6 +1001,7 @@ int timefield3d_clear_probes(timefield3d psi)
     cudaFree(g->d_probes); cudaFree(g->d_probe_buf); cudaFree(g->d_probe_count);
     g->d_probes = nullptr; g->d_probe_buf = nullptr; g->d_probe_count = nullptr;
     g->probes.clear();
+    g->probes_interior = true;
     g->probe_cap = 0;
     g->version++;
     return FDTD_OK;

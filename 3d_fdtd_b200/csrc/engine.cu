@@ -130,10 +130,16 @@ static uint64_t mode_fingerprint(const mode &m)
     // FNV-1a over the dimensions and up to 257 evenly spaced complex entries:
     // catches a mode rescaled in place (mode_smul) or replaced at the same
     // address, at O(1) cost per call.
+    // (eight bytes a round: every source and overlap call computes it)
     uint64_t h = 1469598103934665603ull;
     auto mix = [&](const void *p, size_t n) {
         const unsigned char *c = (const unsigned char *)p;
-        for (size_t i = 0; i < n; i++) { h ^= c[i]; h *= 1099511628211ull; }
+        for (; n > 0; c += std::min<size_t>(n, 8), n -= std::min<size_t>(n, 8)) {
+            uint64_t w = 0;
+            memcpy(&w, c, std::min<size_t>(n, 8));
+            h = (h ^ w) * 1099511628211ull;
+            h ^= h >> 29;   // a word's high bits reach the low ones
+        }
     };
     mix(&m.i, sizeof m.i);
     mix(&m.j, sizeof m.j);
@@ -356,7 +362,7 @@ Grid::~Grid()
         for (int m = 0; m < 6; m++) dfree(sig[m]);
         for (auto &p : planes) dfree(p.p);
         for (auto p : plane_pool) dfree(p);
-        dfree(d_step); dfree(d_done); dfree(d_jobs); dfree(d_job1); dfree(d_partials); dfree(d_inst);
+        dfree(d_step); dfree(d_done); dfree(d_jobs); dfree(d_partials);
         dfree(wave.d_items); dfree(wave.d_cnt); dfree(wave.d_part); dfree(wave.d_ring);
         for (int s = 0; s < 2; s++)
             for (int e = 0; e < 2; e++)
@@ -570,8 +576,6 @@ bool grid_ensure_device(Grid *g)
         CK(cudaMallocHost(&g->h_inst, sizeof(double2)));
         CK(cudaMallocHost(&g->h_err, sizeof(int)));
         if (!dalloc(&g->d_err, sizeof(int), g->st)) return false;
-        if (!dalloc(&g->d_inst, sizeof(double2), g->st)) return false;
-        if (!dalloc(&g->d_job1, sizeof(OverlapJob), g->st)) return false;
         g->jobs_cap = 8;
         if (!dalloc(&g->d_jobs, g->jobs_cap * sizeof(OverlapJob), g->st, false)) return false;
         const int parts = overlap_parts((long long)g->nx * g->ny);
@@ -891,18 +895,34 @@ void grid_zero(Grid *g)
 // ---------------------------------------------------------------------------
 // the step
 // ---------------------------------------------------------------------------
-template <typename T> static bool step_split(Grid *g, double dt)
+// extras: enqueue_after_step follows
+template <typename T> static bool step_split(Grid *g, double dt, bool extras)
 {
     GridView<T> v = view<T>(g, g->cur);
     CpmlView<T> c = cpml_view<T>(g, g->cur);
     SourcePlanes s = source_table(g);
     const T tdt = (T)dt, div = (T)(1 / (g->dx)), tdx = (T)g->dx;
     const bool cpml = g->boundary == FDTD_BOUNDARY_CPML;
-    if (g->boundary == FDTD_BOUNDARY_MUR) launch_save_shell<T>(v, g->st);
-    launch_update_E<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_e, cpml, false, g->st);
-    if (g->boundary == FDTD_BOUNDARY_MUR) launch_mur<T>(v, tdt, tdx, 1, 0, g->nz, g->st);
-    launch_update_H<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_m, g->mu_nonunit, cpml, false, g->st);
-    if (g->boundary == FDTD_BOUNDARY_MUR) launch_mur<T>(v, tdt, tdx, 0, 0, g->nz, g->st);
+    const bool mur = g->boundary == FDTD_BOUNDARY_MUR;
+    launch_update_E<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_e, cpml, false, mur, g->st);
+    launch_update_H<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_m, g->mu_nonunit, cpml, false, mur, tdx, g->st);
+    if (mur) {
+        // a step by itself ends with this launch when nothing reads the counter after it
+        StepEnd end{};
+        const bool own = extras && !g->in_run && g->njobs == 0 && g->binds.empty();
+        if (own) end.step = g->d_step;
+        if (own && g->probes_interior && !g->probes.empty()) {
+            end.probes = g->d_probes;
+            end.np = (int)g->probes.size();
+            end.buf = g->d_probe_buf;
+            end.cap = g->probe_cap;
+            end.count = g->d_probe_count;
+        }
+        launch_mur_step<T>(v, tdt, tdx, end, g->st);
+        CKL("step");
+        g->step_ended = own;
+        g->probes_done = end.np > 0;
+    }
     CKL("step");
     return true;
 }
@@ -993,7 +1013,9 @@ bool enqueue_after_step(Grid *g, double dt)
 {
     const void *const *fp = (const void *const *)g->d_fptr[g->cur];
     const bool f64 = g->prec == FDTD_F64;
-    if (!g->probes.empty()) {
+    const bool ended = g->step_ended, probed = g->probes_done;   // by the step's last launch
+    g->step_ended = g->probes_done = false;
+    if (!g->probes.empty() && !probed) {
         if (f64) launch_probes<double>((const double *const *)fp, g->d_probes, (int)g->probes.size(), g->d_probe_buf, g->probe_cap, g->d_probe_count, g->st);
         else launch_probes<float>((const float *const *)fp, g->d_probes, (int)g->probes.size(), g->d_probe_buf, g->probe_cap, g->d_probe_count, g->st);
     }
@@ -1014,7 +1036,8 @@ bool enqueue_after_step(Grid *g, double dt)
         if (!td) continue;
         if (!enqueue_taper_store(td, g, b.which, 0, g->d_step, b.t0, b.dir)) return false;
     }
-    if (!g->in_run) {
+    if (ended) {
+    } else if (!g->in_run) {
         launch_step_advance(g->d_step, g->st);
     } else {
         // overlaps of this step, scheduled source of the next, counter: one launch
@@ -1104,11 +1127,11 @@ bool enqueue_step(Grid *g, double dt, bool with_extras)
     // External: captured as an event-record node whose timestamp the host can
     // read after a replay (a plain record during capture is only a dependency)
     if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step], g->st, cudaEventRecordExternal));
-    if (g->prec == FDTD_F64) ok = step_split<double>(g, dt);
+    if (g->prec == FDTD_F64) ok = step_split<double>(g, dt, with_extras);
     else if (stream_path(g)) ok = step_stream(g, dt);
     else if (fused_path(g)) ok = step_fused(g, dt);
     else if (fast32_path(g)) ok = step_flat(g, dt);
-    else ok = step_split<float>(g, dt);
+    else ok = step_split<float>(g, dt, with_extras);
     if (!ok) return false;
     if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step + 1], g->st, cudaEventRecordExternal));
     return with_extras ? enqueue_after_step(g, dt) : true;

@@ -140,10 +140,8 @@ struct Grid {
     OverlapJob *d_jobs = nullptr;       // monitors
     int jobs_cap = 0, njobs = 0;
     long long job_cells = 0;        // largest overlap window of the jobs
-    OverlapJob *d_job1 = nullptr;       // single compat overlap
     double2 *d_partials = nullptr;
-    double2 *d_inst = nullptr;
-    double2 *h_inst = nullptr;          // pinned
+    double2 *h_inst = nullptr;          // pinned, written by the overlap kernel
     std::vector<Monitor> monitors;
 
     // probes
@@ -152,6 +150,8 @@ struct Grid {
     double *d_probe_buf = nullptr;
     int *d_probe_count = nullptr;
     int probe_cap = 0;
+    bool probes_interior = true;        // no probe on the shell (a Mur step's last launch may record them)
+    bool step_ended = false, probes_done = false;   // the step's last launch advanced the counter / recorded them
 
     // running DFTs: whole grid, and y-slices by index
     double2 *d_dft_full = nullptr;

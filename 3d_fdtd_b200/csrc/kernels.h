@@ -109,12 +109,24 @@ struct ProbeJob {
 // yee_split.cu
 template <typename T>
 void launch_update_E(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor, int k_lo,
-                     int k_hi, bool sig, bool cpml, bool expl, cudaStream_t st);
+                     int k_hi, bool sig, bool cpml, bool expl, bool snapshot, cudaStream_t st);
 template <typename T>
 void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor, int k_lo,
-                     int k_hi, bool sig, bool mu, bool cpml, bool expl, cudaStream_t st);
+                     int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, T dx, cudaStream_t st);
 template <typename T> void launch_save_shell(const GridView<T> &g, cudaStream_t st);
 template <typename T> void launch_mur(const GridView<T> &g, T dt, T dx, int efield, int ks, int ke, cudaStream_t st);
+// what the last launch of a step also does: record the probes, advance the counter (null: not)
+struct StepEnd {
+    const ProbeJob *probes;
+    int np;
+    double *buf;
+    int cap;
+    int *count;
+    long long *step;
+};
+// The Mur faces of a whole step: launch_update_E with `snapshot`, launch_update_H
+// with `faces` (E's faces), launch_mur_step (H's)
+template <typename T> void launch_mur_step(const GridView<T> &g, T dt, T dx, const StepEnd &end, cudaStream_t st);
 template <typename T> void launch_aos_to_soa(const double *aos, T *const d[6], long long n, cudaStream_t st);
 template <typename T> void launch_soa_to_aos(double *aos, T *const s[6], long long n, cudaStream_t st);
 
@@ -336,6 +348,11 @@ void launch_step_tail(TailArgs a, cudaStream_t st);
 void launch_set_value(float *p, long long idx, float v, cudaStream_t st);
 int overlap_parts(long long cells);
 // cells: the largest overlap window (win.wni * win.wnj) of the jobs
+// one job's instantaneous overlap, written to *out (which the host may read after
+// a synchronisation: pinned memory); done: 0 between launches
+template <typename T>
+void launch_overlap_now(const T *const *f_dev, int nx, int ny, const OverlapJob &job, double2 *partials, unsigned *done,
+                        double scale, double2 *out, cudaStream_t st);
 template <typename T>
 void launch_overlap(const T *const *f_dev, int nx, int ny, const OverlapJob *jobs_dev, int njobs, long long cells,
                     double2 *partials, double scale, double dt, const long long *step, int step_offset,

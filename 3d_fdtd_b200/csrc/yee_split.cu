@@ -7,22 +7,155 @@
 // reference's (same operations, same order, no FMA).  It also carries the
 // CPML terms for grids that use FP64 or the non-fused FP32 path.
 //
-// Thread layout: a 32 x 4 block of (x, y) columns; each thread walks a chunk
-// of z planes, carrying the previous plane's H (E pass) or next plane's E
-// (H pass) in registers so that the z-neighbour is read once.
+// Thread layout: one thread a cell, a block 256 consecutive cells of a plane
+// (x fastest), every load of a cell issued before its arithmetic and its
+// stores.  Both updates are bound by memory: E reads E, H and ep and writes E (84
+// B a cell in FP64), H reads both and writes H (72 B).  A thread used to walk
+// 16 planes to keep the z neighbour in a register; its loads then waited for the
+// previous plane's stores (the arrays may alias), one memory latency a plane,
+// and a 64^3 grid had 128 blocks.  With a thread a cell the z and y neighbours
+// come from L2: FP64 steps of the 200 x 160 x 400 grid with a 12-cell CPML went
+// from 0.85 to 0.48 ms (the cells in no slab move 4.8 TB/s in E, 5.5 in H), and of
+// a 64^3 grid with the Mur boundary from 104 to 25 us.
+// FP64 divisions cost as much as a third of the traffic: a cell whose three
+// permittivities are equal (every rasteriser writes them so) takes its
+// coefficient once.
 #include "common.cuh"
 #include "kernels.h"
 
+#include <algorithm>
+
 namespace fdtd {
 
-constexpr int kBX = 32, kBY = 4, kZChunk = 16;
+constexpr int kCellThreads = 256;
+// cell index within one array: a grid's device arrays take more than 100 B a
+// cell, so 2^31 cells do not fit the device
+using cell_t = unsigned;
+
+// Programmatic dependent launch: wait for the previous kernel's results, and let
+// the next one's blocks be set up meanwhile (they wait in turn).  PART 2 of an
+// update does not depend on PART 1, only on what PART 1 waited for before it let
+// this launch start: it works at once and waits for PART 1 at its end, so that
+// whoever waits for it waits for both.
+template <int PART> __device__ __forceinline__ void cell_prologue()
+{
+    if (PART == 2) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <int PART> __device__ __forceinline__ void cell_epilogue()
+{
+    if (PART != 2) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// the source plane at k (component-major), or null
+__device__ __forceinline__ const float *src_of(const SourcePlanes &s, int k)
+{
+    const float *p = nullptr;
+#pragma unroll
+    for (int t = kMaxSourcePlanes - 1; t >= 0; t--)
+        if (t < s.n && s.k[t] == k) p = s.p[t];
+    return p;
+}
+
+// ---------------------------------------------------------------------------
+// The Mur faces (see k_mur) of a whole step, every shell cell at once.  Face f (order x0,
+// y0, z0, xE, yE, zE) sets a cell's tangential components from its old value,
+// the inner neighbour's old value and the neighbour's value at that time.  A
+// component is set by the faces of the two other axes only, so a cell's final
+// value comes from the last of at most two faces it lies on, and where it lies
+// on two, the neighbour's value at that time is what the earlier one gave it.
+// Both read only cells no face sets for that component (the interior's new
+// values) and the snapshot: no order between threads is needed, and the values
+// are the sequential order's bit for bit.
+// Needs g.old to be the snapshot of this step, taken before its E update (the
+// public boundary calls may pass another: k_mur keeps the order with barriers).
+// One block a plane walked its faces one after another, and the first and last
+// block a whole z face: 18.9 us for the E faces of a 64^3 grid and as much for
+// H's, and 24 us for the snapshot; as threads of the E and H updates, and in one
+// short launch after them, they are part of the 25 us of such a step.
+// ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ T mur_scalar(const GridView<T> &g, int efield, int c, int axis, long long q, T dt, T dx)
+{
+    using A = Ar<T>;
+    const int t = 3 - axis - c;
+    const T ep = efield ? (T)g.ep[c][q] : (T)g.ep[t][q];
+    const T mu = efield ? (T)g.mu[t][q] : (T)g.mu[c][q];
+    const T sdt = A::mul(A::div((T)1, A::sqrt_(A::mul(ep, mu))), dt);
+    return A::div(A::sub(sdt, dx), A::add(sdt, dx));
+}
 
 template <typename T>
-__device__ __forceinline__ T src_at(const SourcePlanes &s, int k, int m, long long nxy, long long ij)
+__device__ __forceinline__ T mur_value(T inner_old, T scalar, T inner, T own_old)
 {
-    for (int t = 0; t < s.n; t++)
-        if (s.k[t] == k) return (T)s.p[t][m * nxy + ij];
-    return (T)0;
+    using A = Ar<T>;
+    return A::add(inner_old, A::mul(scalar, A::sub(inner, own_old)));
+}
+
+// cell number u of the shell: planes 0 and nz-1 whole, then the ring of the others
+__device__ __forceinline__ void shell_cell(long long u, int nx, int ny, int nz, int &i, int &j, int &k)
+{
+    const long long nxy = (long long)nx * ny;
+    if (u < 2 * nxy) {
+        k = u < nxy ? 0 : nz - 1;
+        const unsigned t = (unsigned)(u < nxy ? u : u - nxy);
+        j = (int)(t / (unsigned)nx);
+        i = (int)(t - (unsigned)j * nx);
+        return;
+    }
+    const unsigned ring = 2u * nx + 2u * (ny - 2);
+    const unsigned long long v = (unsigned long long)(u - 2 * nxy);
+    const unsigned p = (unsigned)(v / ring), r = (unsigned)(v - (unsigned long long)p * ring);
+    k = 1 + (int)p;
+    if (r < 2u * nx) {
+        j = r < (unsigned)nx ? 0 : ny - 1;
+        i = (int)(r < (unsigned)nx ? r : r - nx);
+    } else {
+        j = 1 + (int)((r - 2u * nx) >> 1);
+        i = (r & 1u) ? nx - 1 : 0;   // 2 nx is even
+    }
+}
+
+// cells of the shell
+__host__ __device__ __forceinline__ long long mur_cells(int nx, int ny, int nz)
+{
+    return 2LL * nx * ny + (nz - 2LL) * (2LL * nx + 2LL * (ny - 2));
+}
+
+// E (efield) or H of shell cell u
+template <typename T>
+__device__ __forceinline__ void mur_shell_cell(const GridView<T> &g, long long u, T dt, T dx, int efield)
+{
+    int i, j, k;
+    shell_cell(u, g.nx, g.ny, g.nz, i, j, k);
+    const long long nxy = (long long)g.nx * g.ny;
+    const long long q = i + (long long)g.nx * j + nxy * k;
+    // per axis: the face the cell lies on, in the faces' order, or -1, and the step inwards
+    const int fx = i == 0 ? 0 : (i == g.nx - 1 ? 3 : -1);
+    const int fy = j == 0 ? 1 : (j == g.ny - 1 ? 4 : -1);
+    const int fz = k == 0 ? 2 : (k == g.nz - 1 ? 5 : -1);
+    const long long dx_ = i == 0 ? 1 : -1, dy_ = j == 0 ? g.nx : -(long long)g.nx, dz_ = k == 0 ? nxy : -nxy;
+    auto component = [&](int c, int a, int fa, long long da, int b, int fb, long long db) {
+        if (fa < 0 && fb < 0) return;
+        const bool a_last = fa > fb;
+        const long long ql = q + (a_last ? da : db);
+        const int m = efield ? c : 3 + c;
+        const T *f = g.f[m], *old = g.old[m];
+        T inner;
+        if ((a_last ? fb : fa) >= 0) {
+            const long long qf = ql + (a_last ? db : da);
+            inner = mur_value(old[qf], mur_scalar(g, efield, c, a_last ? b : a, ql, dt, dx), f[qf], old[ql]);
+        } else {
+            inner = f[ql];
+        }
+        g.f[m][q] = mur_value(old[ql], mur_scalar(g, efield, c, a_last ? a : b, q, dt, dx), inner, old[q]);
+    };
+    component(0, 1, fy, dy_, 2, fz, dz_);
+    component(1, 0, fx, dx_, 2, fz, dz_);
+    component(2, 0, fx, dx_, 1, fy, dy_);
 }
 
 // ---------------------------------------------------------------------------
@@ -30,95 +163,247 @@ __device__ __forceinline__ T src_at(const SourcePlanes &s, int k, int m, long lo
 // (timefield3d.c:1759-1837); explicit form: timefield3d_apply_E_timestep
 // (timefield3d.c:1607-1677).
 // ---------------------------------------------------------------------------
-template <typename T, bool SIG, bool CPML, bool EXPL>
-__global__ void __launch_bounds__(kBX *kBY)
-k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, int k_lo, int k_hi)
+// update coefficients of one E component: out = main (keep e + curl - J)
+template <typename T, bool SIG> __device__ __forceinline__ void e_coeffs(T ep, T sig, T dt, T &main, T &keep)
 {
     using A = Ar<T>;
-    const int i = blockIdx.x * kBX + threadIdx.x;
-    const int j = blockIdx.y * kBY + threadIdx.y;
-    if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2) return;
-    const long long nxy = (long long)g.nx * g.ny;
-    const long long ij = i + (long long)g.nx * j;
-    int k0 = max(k_lo, 1) + blockIdx.z * kZChunk;
-    int k1 = min(min(k_hi, g.nz - 1), k0 + kZChunk);
-    if (k0 >= k1) return;
-    const T *Hx = g.f[3], *Hy = g.f[4], *Hz = g.f[5];
-    long long q = ij + nxy * k0;
-    T hx_m = Hx[q - nxy], hy_m = Hy[q - nxy];
-    for (int k = k0; k < k1; k++, q += nxy) {
-        T hx = Hx[q], hy = Hy[q], hz = Hz[q];
-        T dHz_dy = A::sub(hz, Hz[q - g.nx]);
-        T dHy_dz = A::sub(hy, hy_m);
-        T dHx_dz = A::sub(hx, hx_m);
-        T dHz_dx = A::sub(hz, Hz[q - 1]);
-        T dHy_dx = A::sub(hy, Hy[q - 1]);
-        T dHx_dy = A::sub(hx, Hx[q - g.nx]);
-        hx_m = hx;
-        hy_m = hy;
-        T curl_x, curl_y, curl_z;
-        if (!CPML) {
-            curl_x = A::mul(divisor, A::sub(dHz_dy, dHy_dz));
-            curl_y = A::mul(divisor, A::sub(dHx_dz, dHz_dx));
-            curl_z = A::mul(divisor, A::sub(dHy_dx, dHx_dy));
-        } else {
-            const int L = c.L;
-            int sx = slab_local(i, g.nx, L), sy = slab_local(j, g.ny, L), sz = slab_local(k, g.nz, L);
-            T kx = sx >= 0 ? c.prof[2][0][i] : (T)1;
-            T ky = sy >= 0 ? c.prof[2][1][j] : (T)1;
-            T kz = sz >= 0 ? c.prof[2][2][k] : (T)1;
-            T pxy = 0, pxz = 0, pyx = 0, pyz = 0, pzx = 0, pzy = 0;
-            if (sx >= 0) {
-                long long s = sx + 2LL * L * (j + (long long)g.ny * k);
-                T b = c.prof[0][0][i], a = c.prof[1][0][i];
-                pyx = A::add(A::mul(b, c.psi[0][0][s]), A::mul(a, A::mul(dHz_dx, divisor)));
-                pzx = A::add(A::mul(b, c.psi[0][1][s]), A::mul(a, A::mul(dHy_dx, divisor)));
-                c.psi[0][0][s] = pyx;
-                c.psi[0][1][s] = pzx;
+    const T r = A::div(ep, dt);
+    if (SIG) {
+        main = A::div((T)1, A::add(r, A::mul((T)0.5, sig)));
+        keep = A::sub(r, A::mul((T)0.5, sig));
+    } else {
+        main = A::div((T)1, r);
+        keep = r;
+    }
+}
+
+// CPML state of one cell and field: slab-local indices, the auxiliaries of the
+// slabs it lies in (else 0) and their profiles (else b = a = 0, 1/kappa = 1)
+template <typename T> struct CellCpml {
+    int sx, sy, sz;
+    cell_t ox, oy, oz;
+    T px0, px1, py0, py1, pz0, pz1;
+    T bx, ax, kx, by, ay, ky, bz, az, kz;
+};
+
+// w: 0 for E, 1 for H
+template <typename T>
+__device__ __forceinline__ void cpml_load(CellCpml<T> &p, const CpmlView<T> &c, int nx, int ny, int nz, int i, int j,
+                                          int k, cell_t ij, cell_t nxy, int w)
+{
+    const int L = c.L;
+    p.sx = slab_local(i, nx, L);
+    p.sy = slab_local(j, ny, L);
+    p.sz = slab_local(k, nz, L);
+    p.px0 = p.px1 = p.py0 = p.py1 = p.pz0 = p.pz1 = (T)0;
+    p.bx = p.ax = p.by = p.ay = p.bz = p.az = (T)0;
+    p.kx = p.ky = p.kz = (T)1;
+    if (p.sx >= 0) {
+        p.ox = (cell_t)p.sx + (cell_t)(2 * L) * ((cell_t)j + (cell_t)ny * (cell_t)k);
+        p.px0 = c.psi[0][2 * w][p.ox];
+        p.px1 = c.psi[0][2 * w + 1][p.ox];
+        p.bx = c.prof[3 * w][0][i];
+        p.ax = c.prof[3 * w + 1][0][i];
+        p.kx = c.prof[3 * w + 2][0][i];
+    }
+    if (p.sy >= 0) {
+        p.oy = (cell_t)i + (cell_t)nx * (cell_t)(p.sy + 2 * L * k);
+        p.py0 = c.psi[1][2 * w][p.oy];
+        p.py1 = c.psi[1][2 * w + 1][p.oy];
+        p.by = c.prof[3 * w][1][j];
+        p.ay = c.prof[3 * w + 1][1][j];
+        p.ky = c.prof[3 * w + 2][1][j];
+    }
+    if (p.sz >= 0) {
+        p.oz = ij + nxy * (cell_t)p.sz;
+        p.pz0 = c.psi[2][2 * w][p.oz];
+        p.pz1 = c.psi[2][2 * w + 1][p.oz];
+        p.bz = c.prof[3 * w][2][k];
+        p.az = c.prof[3 * w + 1][2][k];
+        p.kz = c.prof[3 * w + 2][2][k];
+    }
+}
+
+// the curl with its CPML terms; dU_dv: differences as the plain curl uses them
+template <typename T>
+__device__ __forceinline__ void cpml_curl3(CellCpml<T> &p, T divisor, T dz_dy, T dy_dz, T dx_dz, T dz_dx, T dy_dx,
+                                           T dx_dy, T curl[3])
+{
+    using A = Ar<T>;
+    if (p.sx >= 0) {
+        p.px0 = A::add(A::mul(p.bx, p.px0), A::mul(p.ax, A::mul(dz_dx, divisor)));
+        p.px1 = A::add(A::mul(p.bx, p.px1), A::mul(p.ax, A::mul(dy_dx, divisor)));
+    }
+    if (p.sy >= 0) {
+        p.py0 = A::add(A::mul(p.by, p.py0), A::mul(p.ay, A::mul(dz_dy, divisor)));
+        p.py1 = A::add(A::mul(p.by, p.py1), A::mul(p.ay, A::mul(dx_dy, divisor)));
+    }
+    if (p.sz >= 0) {
+        p.pz0 = A::add(A::mul(p.bz, p.pz0), A::mul(p.az, A::mul(dy_dz, divisor)));
+        p.pz1 = A::add(A::mul(p.bz, p.pz1), A::mul(p.az, A::mul(dx_dz, divisor)));
+    }
+    curl[0] = A::add(A::mul(divisor, A::sub(A::mul(dz_dy, p.ky), A::mul(dy_dz, p.kz))), A::sub(p.py0, p.pz0));
+    curl[1] = A::add(A::mul(divisor, A::sub(A::mul(dx_dz, p.kz), A::mul(dz_dx, p.kx))), A::sub(p.pz1, p.px0));
+    curl[2] = A::add(A::mul(divisor, A::sub(A::mul(dy_dx, p.kx), A::mul(dx_dy, p.ky))), A::sub(p.px1, p.py1));
+}
+
+template <typename T>
+__device__ __forceinline__ void cpml_store(const CellCpml<T> &p, const CpmlView<T> &c, int w)
+{
+    if (p.sx >= 0) {
+        c.psi[0][2 * w][p.ox] = p.px0;
+        c.psi[0][2 * w + 1][p.ox] = p.px1;
+    }
+    if (p.sy >= 0) {
+        c.psi[1][2 * w][p.oy] = p.py0;
+        c.psi[1][2 * w + 1][p.oy] = p.py1;
+    }
+    if (p.sz >= 0) {
+        c.psi[2][2 * w][p.oz] = p.pz0;
+        c.psi[2][2 * w + 1][p.oz] = p.pz1;
+    }
+}
+
+// The cells of a launch.  Without CPML: interior cells of planes [k_lo, k_hi)
+// (every cell with a snapshot), a block's 256 consecutive in a plane.  A CPML
+// grid's step takes two launches, PART 1 the cells in no slab and PART 2 those
+// in one: the plain update needs 64 registers a thread and the CPML one 80 to
+// 92, and at two or three blocks an SM the loads in flight do not cover their
+// latency (FP64 E and H of the 200 x 160 x 400 grid: 373 and 307 us in one launch
+// each, 279 and 200 in two).
+// PART 0: both, for calls on a range of planes.
+struct CellRange {
+    int k_lo, k_hi;
+    int x0, y0, w, h;      // columns and rows of a plane: [x0, x0 + w) x [y0, y0 + h)
+    int L;                 // PART 2: slab thickness
+};
+
+// false: no cell of this launch
+template <int PART>
+__device__ __forceinline__ bool cell_of(const CellRange &r, int nx, int ny, int nz, unsigned t, int slot, int &i, int &j,
+                                        int &k)
+{
+    if (PART != 2) {
+        if (t >= (unsigned)r.w * (unsigned)r.h) return false;
+        const int y = (int)(t / (unsigned)r.w);
+        i = r.x0 + (int)(t - (unsigned)y * (unsigned)r.w);
+        j = r.y0 + y;
+        k = r.k_lo + slot;
+        return true;
+    }
+    // cells in one row: the 2L - 2 updated planes of the z slabs, whole, then of
+    // each middle plane the 2L - 2 rows of the y slabs and, in the other rows, the
+    // 2L - 2 columns of the x slabs
+    const unsigned S = (unsigned)r.L - 1, W = (unsigned)nx - 2, H = (unsigned)ny - 2, mid = (unsigned)(ny - 2 * r.L);
+    const unsigned plane = W * H, zcells = 2 * S * plane;
+    if (t < zcells) {
+        const unsigned z = t / plane;
+        t -= z * plane;
+        const unsigned y = t / W;
+        k = (int)(z < S ? 1 + z : (unsigned)(nz - r.L) + z - S);
+        j = 1 + (int)y;
+        i = 1 + (int)(t - y * W);
+        return true;
+    }
+    t -= zcells;
+    const unsigned rows = 2 * S * W, ring = rows + 2 * S * mid;
+    const unsigned z = t / ring;
+    if (z >= (unsigned)(nz - 2 * r.L)) return false;
+    t -= z * ring;
+    k = r.L + (int)z;
+    if (t < rows) {
+        const unsigned y = t / W;
+        j = (int)(y < S ? 1 + y : (unsigned)(ny - r.L) + y - S);
+        i = 1 + (int)(t - y * W);
+        return true;
+    }
+    t -= rows;
+    const unsigned y = t / (2 * S), x = t - y * (2 * S);
+    j = r.L + (int)y;
+    i = (int)(x < S ? 1 + x : (unsigned)(nx - r.L) + x - S);
+    return true;
+}
+
+// slots (planes) and cells of a slot of a launch
+static void cell_extent(const CellRange &r, int nx, int ny, int nz, int part, int &slots, long long &cells)
+{
+    if (part != 2) {
+        slots = r.k_hi - r.k_lo;
+        cells = (long long)r.w * r.h;
+        return;
+    }
+    const long long S = r.L - 1, W = nx - 2, H = ny - 2;
+    slots = 1;
+    cells = 2 * S * W * H + (nz - 2LL * r.L) * (2 * S * W + 2 * S * (ny - 2LL * r.L));
+}
+
+// SNAP: the launch covers every cell and first copies the 2-cell shell of all
+// six components to g.old (timefield3d_update_old_edge_fields,
+// timefield3d.c:246-346): the Mur step's snapshot, taken while the cell is in
+// registers instead of in a launch of its own
+template <typename T, bool SIG, bool CPML, bool EXPL, bool SNAP, int PART>
+__global__ void __launch_bounds__(kCellThreads, CPML ? 3 : 4)
+k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, CellRange r, int slots)
+{
+    using A = Ar<T>;
+    cell_prologue<PART>();
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const cell_t nxy = (cell_t)nx * (cell_t)ny;
+    for (int slot = blockIdx.y; slot < slots; slot += gridDim.y) {
+        int i, j, k;
+        if (!cell_of<PART>(r, nx, ny, nz, blockIdx.x * (unsigned)kCellThreads + threadIdx.x, slot, i, j, k)) continue;
+        const cell_t ij = (cell_t)i + (cell_t)nx * (cell_t)j, q = ij + nxy * (cell_t)k;
+        T e[3];
+        if (SNAP) {
+            const bool shell = i <= 1 || i >= nx - 2 || j <= 1 || j >= ny - 2 || k <= 1 || k >= nz - 2;
+            if (shell) {
+#pragma unroll
+                for (int m = 0; m < 6; m++) g.old[m][q] = g.f[m][q];
             }
-            if (sy >= 0) {
-                long long s = i + (long long)g.nx * (sy + 2LL * L * k);
-                T b = c.prof[0][1][j], a = c.prof[1][1][j];
-                pxy = A::add(A::mul(b, c.psi[1][0][s]), A::mul(a, A::mul(dHz_dy, divisor)));
-                pzy = A::add(A::mul(b, c.psi[1][1][s]), A::mul(a, A::mul(dHx_dy, divisor)));
-                c.psi[1][0][s] = pxy;
-                c.psi[1][1][s] = pzy;
-            }
-            if (sz >= 0) {
-                long long s = ij + nxy * sz;
-                T b = c.prof[0][2][k], a = c.prof[1][2][k];
-                pxz = A::add(A::mul(b, c.psi[2][0][s]), A::mul(a, A::mul(dHy_dz, divisor)));
-                pyz = A::add(A::mul(b, c.psi[2][1][s]), A::mul(a, A::mul(dHx_dz, divisor)));
-                c.psi[2][0][s] = pxz;
-                c.psi[2][1][s] = pyz;
-            }
-            curl_x = A::add(A::mul(divisor, A::sub(A::mul(dHz_dy, ky), A::mul(dHy_dz, kz))), A::sub(pxy, pxz));
-            curl_y = A::add(A::mul(divisor, A::sub(A::mul(dHx_dz, kz), A::mul(dHz_dx, kx))), A::sub(pyz, pyx));
-            curl_z = A::add(A::mul(divisor, A::sub(A::mul(dHy_dx, kx), A::mul(dHx_dy, ky))), A::sub(pzx, pzy));
+            if (i < 1 || i > nx - 2 || j < 1 || j > ny - 2 || k < 1 || k > nz - 2) continue;
         }
-        T curl[3] = {curl_x, curl_y, curl_z};
+        const float *sp = src_of(src, k);
+        const T hx = g.f[3][q], hy = g.f[4][q], hz = g.f[5][q];
+        const T hx_j = g.f[3][q - nx], hz_j = g.f[5][q - nx];
+        const T hx_k = g.f[3][q - nxy], hy_k = g.f[4][q - nxy];
+        const T hy_i = g.f[4][q - 1], hz_i = g.f[5][q - 1];
+        T ep[3], sig[3];
 #pragma unroll
         for (int m = 0; m < 3; m++) {
-            T e = g.f[m][q];
-            T ep = (T)g.ep[m][q];
-            T sig = SIG ? (T)g.sig[m][q] : (T)0;
-            T J = src_at<T>(src, k, m, nxy, ij);
-            T out;
-            if (EXPL) {
-                T Jt = A::add(J, A::mul(e, sig));
-                out = A::add(e, A::div(A::mul(dt, A::sub(curl[m], Jt)), ep));
-            } else if (SIG) {
-                T main_coeff = A::div((T)1, A::add(A::div(ep, dt), A::mul((T)0.5, sig)));
-                T e_coeff = A::sub(A::div(ep, dt), A::mul((T)0.5, sig));
-                out = A::mul(main_coeff, A::sub(A::add(A::mul(e_coeff, e), curl[m]), J));
-            } else {
-                T e_coeff = A::div(ep, dt);
-                T main_coeff = A::div((T)1, e_coeff);
-                out = A::mul(main_coeff, A::sub(A::add(A::mul(e_coeff, e), curl[m]), J));
-            }
-            g.f[m][q] = out;
+            e[m] = g.f[m][q];
+            ep[m] = (T)g.ep[m][q];
+            sig[m] = SIG ? (T)g.sig[m][q] : (T)0;
         }
+        CellCpml<T> p;
+        if (CPML) cpml_load(p, c, nx, ny, nz, i, j, k, ij, nxy, 0);
+        const T dHz_dy = A::sub(hz, hz_j), dHy_dz = A::sub(hy, hy_k), dHx_dz = A::sub(hx, hx_k);
+        const T dHz_dx = A::sub(hz, hz_i), dHy_dx = A::sub(hy, hy_i), dHx_dy = A::sub(hx, hx_j);
+        T curl[3];
+        if (CPML) {
+            cpml_curl3(p, divisor, dHz_dy, dHy_dz, dHx_dz, dHz_dx, dHy_dx, dHx_dy, curl);
+        } else {
+            curl[0] = A::mul(divisor, A::sub(dHz_dy, dHy_dz));
+            curl[1] = A::mul(divisor, A::sub(dHx_dz, dHz_dx));
+            curl[2] = A::mul(divisor, A::sub(dHy_dx, dHx_dy));
+        }
+        T main = 0, keep = 0;
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const T J = sp ? (T)sp[m * nxy + ij] : (T)0;
+            if (EXPL) {
+                const T Jt = A::add(J, A::mul(e[m], sig[m]));
+                e[m] = A::add(e[m], A::div(A::mul(dt, A::sub(curl[m], Jt)), ep[m]));
+            } else {
+                if (m == 0 || ep[m] != ep[m - 1] || (SIG && sig[m] != sig[m - 1]))
+                    e_coeffs<T, SIG>(ep[m], sig[m], dt, main, keep);
+                e[m] = A::mul(main, A::sub(A::add(A::mul(keep, e[m]), curl[m]), J));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 3; m++) g.f[m][q] = e[m];
+        if (CPML) cpml_store(p, c, 0);
     }
+    cell_epilogue<PART>();
 }
 
 // ---------------------------------------------------------------------------
@@ -127,96 +412,82 @@ k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, int 
 // (timefield3d.c:1705-1707); explicit: timefield3d_apply_H_timestep
 // (timefield3d.c:1537-1605).
 // ---------------------------------------------------------------------------
-template <typename T, bool SIG, bool MU, bool CPML, bool EXPL>
-__global__ void __launch_bounds__(kBX *kBY)
-k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, int k_lo, int k_hi)
+// h_coeff, h_main: 1/dt and 1/(1/dt), the coefficients where mu = 1 and no loss
+// MUR: the launch also sets E on the shell (the E faces of the Mur step): slots
+// past the planes are the shell's cells.  An interior cell whose +x, +y or +z
+// neighbour is on the shell needs that face's new E and computes it itself --
+// such a neighbour lies on one face only, and its inner neighbour is the cell --
+// so H waits for no launch of its own between the two.
+template <typename T, bool SIG, bool MU, bool CPML, bool EXPL, int PART, bool MUR>
+__global__ void __launch_bounds__(kCellThreads, CPML ? 3 : 4)
+k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_coeff, T h_main, CellRange r, int slots,
+           T dx)
 {
     using A = Ar<T>;
-    const int i = blockIdx.x * kBX + threadIdx.x;
-    const int j = blockIdx.y * kBY + threadIdx.y;
-    if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2) return;
-    const long long nxy = (long long)g.nx * g.ny;
-    const long long ij = i + (long long)g.nx * j;
-    int k0 = max(k_lo, 1) + blockIdx.z * kZChunk;
-    int k1 = min(min(k_hi, g.nz - 1), k0 + kZChunk);
-    if (k0 >= k1) return;
-    const T *Ex = g.f[0], *Ey = g.f[1], *Ez = g.f[2];
-    long long q = ij + nxy * k0;
-    T ex = Ex[q], ey = Ey[q];
-    for (int k = k0; k < k1; k++, q += nxy) {
-        T ez = Ez[q];
-        T ex_p = Ex[q + nxy], ey_p = Ey[q + nxy];
-        T dEz_dy = A::sub(Ez[q + g.nx], ez);
-        T dEy_dz = A::sub(ey_p, ey);
-        T dEx_dz = A::sub(ex_p, ex);
-        T dEz_dx = A::sub(Ez[q + 1], ez);
-        T dEy_dx = A::sub(Ey[q + 1], ey);
-        T dEx_dy = A::sub(Ex[q + g.nx], ex);
-        ex = ex_p;
-        ey = ey_p;
-        T curl_x, curl_y, curl_z;
-        if (!CPML) {
-            curl_x = A::mul(divisor, A::sub(dEz_dy, dEy_dz));
-            curl_y = A::mul(divisor, A::sub(dEx_dz, dEz_dx));
-            curl_z = A::mul(divisor, A::sub(dEy_dx, dEx_dy));
-        } else {
-            const int L = c.L;
-            int sx = slab_local(i, g.nx, L), sy = slab_local(j, g.ny, L), sz = slab_local(k, g.nz, L);
-            T kx = sx >= 0 ? c.prof[5][0][i] : (T)1;
-            T ky = sy >= 0 ? c.prof[5][1][j] : (T)1;
-            T kz = sz >= 0 ? c.prof[5][2][k] : (T)1;
-            T pxy = 0, pxz = 0, pyx = 0, pyz = 0, pzx = 0, pzy = 0;
-            if (sx >= 0) {
-                long long s = sx + 2LL * L * (j + (long long)g.ny * k);
-                T b = c.prof[3][0][i], a = c.prof[4][0][i];
-                pyx = A::add(A::mul(b, c.psi[0][2][s]), A::mul(a, A::mul(dEz_dx, divisor)));
-                pzx = A::add(A::mul(b, c.psi[0][3][s]), A::mul(a, A::mul(dEy_dx, divisor)));
-                c.psi[0][2][s] = pyx;
-                c.psi[0][3][s] = pzx;
-            }
-            if (sy >= 0) {
-                long long s = i + (long long)g.nx * (sy + 2LL * L * k);
-                T b = c.prof[3][1][j], a = c.prof[4][1][j];
-                pxy = A::add(A::mul(b, c.psi[1][2][s]), A::mul(a, A::mul(dEz_dy, divisor)));
-                pzy = A::add(A::mul(b, c.psi[1][3][s]), A::mul(a, A::mul(dEx_dy, divisor)));
-                c.psi[1][2][s] = pxy;
-                c.psi[1][3][s] = pzy;
-            }
-            if (sz >= 0) {
-                long long s = ij + nxy * sz;
-                T b = c.prof[3][2][k], a = c.prof[4][2][k];
-                pxz = A::add(A::mul(b, c.psi[2][2][s]), A::mul(a, A::mul(dEy_dz, divisor)));
-                pyz = A::add(A::mul(b, c.psi[2][3][s]), A::mul(a, A::mul(dEx_dz, divisor)));
-                c.psi[2][2][s] = pxz;
-                c.psi[2][3][s] = pyz;
-            }
-            curl_x = A::add(A::mul(divisor, A::sub(A::mul(dEz_dy, ky), A::mul(dEy_dz, kz))), A::sub(pxy, pxz));
-            curl_y = A::add(A::mul(divisor, A::sub(A::mul(dEx_dz, kz), A::mul(dEz_dx, kx))), A::sub(pyz, pyx));
-            curl_z = A::add(A::mul(divisor, A::sub(A::mul(dEy_dx, kx), A::mul(dEx_dy, ky))), A::sub(pzx, pzy));
+    cell_prologue<PART>();
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const cell_t nxy = (cell_t)nx * (cell_t)ny;
+    const int shell_slots = MUR ? (int)((mur_cells(nx, ny, nz) + gridDim.x * kCellThreads - 1) /
+                                        (gridDim.x * kCellThreads)) : 0;
+    for (int slot = blockIdx.y; slot < slots + shell_slots; slot += gridDim.y) {
+        int i, j, k;
+        if (MUR && slot >= slots) {
+            const long long u = ((long long)(slot - slots) * gridDim.x + blockIdx.x) * kCellThreads + threadIdx.x;
+            if (u < mur_cells(nx, ny, nz)) mur_shell_cell(g, u, dt, dx, 1);
+            continue;
         }
-        T curl[3] = {curl_x, curl_y, curl_z};
+        if (!cell_of<PART>(r, nx, ny, nz, blockIdx.x * (unsigned)kCellThreads + threadIdx.x, slot, i, j, k)) continue;
+        const cell_t ij = (cell_t)i + (cell_t)nx * (cell_t)j, q = ij + nxy * (cell_t)k;
+        const float *sp = src_of(src, k);
+        const T ex = g.f[0][q], ey = g.f[1][q], ez = g.f[2][q];
+        T ex_j, ez_j, ex_k, ey_k, ey_i, ez_i;
+        auto next = [&](int c, T inner, int axis, cell_t qn, bool face) -> T {
+            return MUR && face ? mur_value(g.old[c][q], mur_scalar(g, 1, c, axis, qn, dt, dx), inner, g.old[c][qn])
+                               : g.f[c][qn];
+        };
+        ex_j = next(0, ex, 1, q + nx, j == ny - 2);
+        ez_j = next(2, ez, 1, q + nx, j == ny - 2);
+        ex_k = next(0, ex, 2, q + nxy, k == nz - 2);
+        ey_k = next(1, ey, 2, q + nxy, k == nz - 2);
+        ey_i = next(1, ey, 0, q + 1, i == nx - 2);
+        ez_i = next(2, ez, 0, q + 1, i == nx - 2);
+        T h[3], mu[3], sig[3];
 #pragma unroll
         for (int m = 0; m < 3; m++) {
-            T h = g.f[3 + m][q];
-            T mu = MU ? (T)g.mu[m][q] : (T)1;
-            T sig = SIG ? (T)g.sig[3 + m][q] : (T)0;
-            T M = src_at<T>(src, k, 3 + m, nxy, ij);
-            if (SIG) M = A::add(M, A::mul(h, sig));
-            T out;
-            if (EXPL) {
-                out = A::sub(h, A::div(A::mul(dt, A::add(curl[m], M)), mu));
-            } else if (SIG) {
-                T main_coeff = A::div((T)1, A::add(A::div(mu, dt), A::mul((T)0.5, sig)));
-                T h_coeff = A::sub(A::div(mu, dt), A::mul((T)0.5, sig));
-                out = A::mul(main_coeff, A::sub(A::sub(A::mul(h_coeff, h), curl[m]), M));
-            } else {
-                T h_coeff = A::div(mu, dt);
-                T main_coeff = A::div((T)1, h_coeff);
-                out = A::mul(main_coeff, A::sub(A::sub(A::mul(h_coeff, h), curl[m]), M));
-            }
-            g.f[3 + m][q] = out;
+            h[m] = g.f[3 + m][q];
+            mu[m] = MU ? (T)g.mu[m][q] : (T)1;
+            sig[m] = SIG ? (T)g.sig[3 + m][q] : (T)0;
         }
+        CellCpml<T> p;
+        if (CPML) cpml_load(p, c, nx, ny, nz, i, j, k, ij, nxy, 1);
+        const T dEz_dy = A::sub(ez_j, ez), dEy_dz = A::sub(ey_k, ey), dEx_dz = A::sub(ex_k, ex);
+        const T dEz_dx = A::sub(ez_i, ez), dEy_dx = A::sub(ey_i, ey), dEx_dy = A::sub(ex_j, ex);
+        T curl[3];
+        if (CPML) {
+            cpml_curl3(p, divisor, dEz_dy, dEy_dz, dEx_dz, dEz_dx, dEy_dx, dEx_dy, curl);
+        } else {
+            curl[0] = A::mul(divisor, A::sub(dEz_dy, dEy_dz));
+            curl[1] = A::mul(divisor, A::sub(dEx_dz, dEz_dx));
+            curl[2] = A::mul(divisor, A::sub(dEy_dx, dEx_dy));
+        }
+        T main = h_main, keep = h_coeff;
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            T M = sp ? (T)sp[(3 + m) * nxy + ij] : (T)0;
+            if (SIG) M = A::add(M, A::mul(h[m], sig[m]));
+            if (EXPL) {
+                h[m] = A::sub(h[m], A::div(A::mul(dt, A::add(curl[m], M)), mu[m]));
+            } else {
+                if ((SIG || MU) && (m == 0 || mu[m] != mu[m - 1] || (SIG && sig[m] != sig[m - 1])))
+                    e_coeffs<T, SIG>(mu[m], sig[m], dt, main, keep);
+                h[m] = A::mul(main, A::sub(A::sub(A::mul(keep, h[m]), curl[m]), M));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 3; m++) g.f[3 + m][q] = h[m];
+        if (CPML) cpml_store(p, c, 1);
     }
+    cell_epilogue<PART>();
 }
 
 // ---------------------------------------------------------------------------
@@ -338,6 +609,25 @@ __global__ void k_mur(GridView<T> g, T dt, T dx, int efield, int ks, int ke)
     }
 }
 
+// H faces of a step, the probes (interior ones: no face sets them) and the step
+// counter
+template <typename T>
+__global__ void __launch_bounds__(kCellThreads) k_mur_step(GridView<T> g, T dt, T dx, StepEnd end)
+{
+    cell_prologue<0>();
+    if (blockIdx.x == gridDim.x - 1) {
+        for (int p = threadIdx.x; p < end.np; p += kCellThreads) {
+            const int n = end.count[p];
+            if (n < end.cap) end.buf[(long long)p * end.cap + n] = (double)g.f[end.probes[p].m][end.probes[p].q];
+            end.count[p] = n + 1;
+        }
+        if (threadIdx.x == 0 && end.step) *end.step += 1;
+        return;
+    }
+    const long long u = blockIdx.x * (long long)kCellThreads + threadIdx.x;
+    if (u < mur_cells(g.nx, g.ny, g.nz)) mur_shell_cell(g, u, dt, dx, 0);
+}
+
 // AoS double (reference layout) -> SoA T, whole grid
 template <typename T>
 __global__ void k_aos_to_soa(const double *aos, T *d0, T *d1, T *d2, T *d3, T *d4, T *d5, long long n)
@@ -364,47 +654,108 @@ __global__ void k_soa_to_aos(double *aos, const T *s0, const T *s1, const T *s2,
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-static dim3 grid_for(int nx, int ny, int k_lo, int k_hi, int nz)
+// launch with a programmatic dependency on the preceding kernel (cell_prologue)
+template <typename... P, typename... A>
+static void launch_cells(void (*k)(P...), dim3 grid, cudaStream_t st, A... args)
 {
-    int a = k_lo < 1 ? 1 : k_lo, b = k_hi > nz - 1 ? nz - 1 : k_hi;
-    int nk = b > a ? b - a : 0;
-    return dim3((nx + kBX - 1) / kBX, (ny + kBY - 1) / kBY, (nk + kZChunk - 1) / kZChunk);
+    note_launch();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kCellThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
+template <typename F> static void for_range(const CellRange &r, int nx, int ny, int nz, int part, F f)
+{
+    int slots;
+    long long cells;
+    cell_extent(r, nx, ny, nz, part, slots, cells);
+    if (slots <= 0 || cells <= 0) return;
+    f(dim3((unsigned)((cells + kCellThreads - 1) / kCellThreads), (unsigned)(slots < 65535 ? slots : 65535)), slots);
+}
+
+// interior cells of planes [k_lo, k_hi), or (snapshot) every cell
+static CellRange cell_range(int nx, int ny, int nz, int k_lo, int k_hi, bool snapshot)
+{
+    if (snapshot) return CellRange{0, nz, 0, 0, nx, ny, 0};
+    return CellRange{k_lo < 1 ? 1 : k_lo, k_hi > nz - 1 ? nz - 1 : k_hi, 1, 1, nx - 2, ny - 2, 0};
+}
+
+// the cells of a CPML grid in no slab
+static CellRange slab_free(int nx, int ny, int nz, int L)
+{
+    return CellRange{L, nz - L, L, L, nx - 2 * L, ny - 2 * L, L};
 }
 
 template <typename T>
 void launch_update_E(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor,
-                     int k_lo, int k_hi, bool sig, bool cpml, bool expl, cudaStream_t st)
+                     int k_lo, int k_hi, bool sig, bool cpml, bool expl, bool snapshot, cudaStream_t st)
 {
-    dim3 grd = grid_for(g.nx, g.ny, k_lo, k_hi, g.nz), blk(kBX, kBY);
-    if (grd.z == 0) return;
-    note_launch();
-    if (expl) k_update_E<T, true, false, true><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi);
-    else if (cpml) {
-        if (sig) k_update_E<T, true, true, false><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi);
-        else k_update_E<T, false, true, false><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi);
-    } else {
-        if (sig) k_update_E<T, true, false, false><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi);
-        else k_update_E<T, false, false, false><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi);
+    const CellRange all = cell_range(g.nx, g.ny, g.nz, k_lo, k_hi, snapshot);
+    const bool whole = cpml && c.L >= 1 && all.k_lo == 1 && all.k_hi == g.nz - 1;
+#define FDTD_E(RANGE, ...)                                                                            \
+    for_range(RANGE, g.nx, g.ny, g.nz, part, [&](dim3 grd, int slots) {                               \
+        launch_cells(k_update_E<T, __VA_ARGS__>, grd, st, g, c, s, dt, divisor, RANGE, slots);        \
+    })
+    int part = 0;
+    if (expl) FDTD_E(all, true, false, true, false, 0);
+    else if (whole) {
+        const CellRange in = slab_free(g.nx, g.ny, g.nz, c.L);
+        part = 1;
+        if (sig) FDTD_E(in, true, false, false, false, 1); else FDTD_E(in, false, false, false, false, 1);
+        part = 2;
+        if (sig) FDTD_E(in, true, true, false, false, 2); else FDTD_E(in, false, true, false, false, 2);
     }
+    else if (cpml) { if (sig) FDTD_E(all, true, true, false, false, 0); else FDTD_E(all, false, true, false, false, 0); }
+    else if (snapshot) { if (sig) FDTD_E(all, true, false, false, true, 0); else FDTD_E(all, false, false, false, true, 0); }
+    else { if (sig) FDTD_E(all, true, false, false, false, 0); else FDTD_E(all, false, false, false, false, 0); }
+#undef FDTD_E
 }
 
 template <typename T>
 void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor,
-                     int k_lo, int k_hi, bool sig, bool mu, bool cpml, bool expl, cudaStream_t st)
+                     int k_lo, int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, T dx, cudaStream_t st)
 {
-    dim3 grd = grid_for(g.nx, g.ny, k_lo, k_hi, g.nz), blk(kBX, kBY);
-    if (grd.z == 0) return;
-    note_launch();
-    if (expl) { k_update_H<T, true, true, false, true><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi); return; }
-#define FDTD_H(SG, MU_, CP) k_update_H<T, SG, MU_, CP, false><<<grd, blk, 0, st>>>(g, c, s, dt, divisor, k_lo, k_hi)
-    if (sig) {
-        if (cpml) FDTD_H(true, true, true); else FDTD_H(true, true, false);
-    } else if (mu) {
-        if (cpml) FDTD_H(false, true, true); else FDTD_H(false, true, false);
-    } else {
-        if (cpml) FDTD_H(false, false, true); else FDTD_H(false, false, false);
+    const CellRange all = cell_range(g.nx, g.ny, g.nz, k_lo, k_hi, false);
+    const T h_coeff = (T)1 / dt, h_main = (T)1 / h_coeff;
+    const bool whole = cpml && c.L >= 1 && all.k_lo == 1 && all.k_hi == g.nz - 1;
+#define FDTD_H(RANGE, ...)                                                                                          \
+    for_range(RANGE, g.nx, g.ny, g.nz, part, [&](dim3 grd, int slots) {                                             \
+        if (faces) grd.y = (unsigned)std::min<long long>(65535, grd.y + mur_cells(g.nx, g.ny, g.nz) / ((long long)grd.x * kCellThreads) + 1); \
+        launch_cells(k_update_H<T, __VA_ARGS__>, grd, st, g, c, s, dt, divisor, h_coeff, h_main, RANGE, slots, dx); \
+    })
+#define FDTD_H3(RANGE, CP, PT, FACES)                                     \
+    do {                                                                  \
+        if (sig) FDTD_H(RANGE, true, true, CP, false, PT, FACES);         \
+        else if (mu) FDTD_H(RANGE, false, true, CP, false, PT, FACES);    \
+        else FDTD_H(RANGE, false, false, CP, false, PT, FACES);           \
+    } while (0)
+    int part = 0;
+    if (expl) FDTD_H(all, true, true, false, true, 0, false);
+    else if (whole) {
+        const CellRange in = slab_free(g.nx, g.ny, g.nz, c.L);
+        part = 1;
+        FDTD_H3(in, false, 1, false);
+        part = 2;
+        FDTD_H3(in, true, 2, false);
     }
+    else if (cpml) FDTD_H3(all, true, 0, false);
+    else if (faces) FDTD_H3(all, false, 0, true);
+    else FDTD_H3(all, false, 0, false);
+#undef FDTD_H3
 #undef FDTD_H
+}
+
+template <typename T> void launch_mur_step(const GridView<T> &g, T dt, T dx, const StepEnd &end, cudaStream_t st)
+{
+    const long long blocks = (mur_cells(g.nx, g.ny, g.nz) + kCellThreads - 1) / kCellThreads + 1;
+    launch_cells(k_mur_step<T>, dim3((unsigned)blocks), st, g, dt, dx, end);
 }
 
 template <typename T>
@@ -444,9 +795,10 @@ void launch_soa_to_aos(double *aos, T *const s[6], long long n, cudaStream_t st)
 
 #define FDTD_INST(T)                                                                                          \
     template void launch_update_E<T>(const GridView<T> &, const CpmlView<T> &, const SourcePlanes &, T, T, int, \
-                                     int, bool, bool, bool, cudaStream_t);                                     \
-    template void launch_update_H<T>(const GridView<T> &, const CpmlView<T> &, const SourcePlanes &, T, T, int, \
                                      int, bool, bool, bool, bool, cudaStream_t);                               \
+    template void launch_mur_step<T>(const GridView<T> &, T, T, const StepEnd &, cudaStream_t);                \
+    template void launch_update_H<T>(const GridView<T> &, const CpmlView<T> &, const SourcePlanes &, T, T, int, \
+                                     int, bool, bool, bool, bool, bool, T, cudaStream_t);                      \
     template void launch_save_shell<T>(const GridView<T> &, cudaStream_t);                                    \
     template void launch_mur<T>(const GridView<T> &, T, T, int, int, int, cudaStream_t);                       \
     template void launch_aos_to_soa<T>(const double *, T *const[6], long long, cudaStream_t);                  \
