@@ -374,6 +374,8 @@ Grid::~Grid()
         delete fmaps[0];
         delete fmaps[1];
         dfree(d_tiles);
+        dfree(d_boxes);
+        dfree(d_maps);
         dfree(d_flag);
         for (auto &mn : monitors) { dfree(mn.d_omega); dfree(mn.d_acc); priv_mode_free(mn.mode_key); }
         dfree(d_probes); dfree(d_probe_buf); dfree(d_probe_count);
@@ -422,13 +424,15 @@ SourcePlanes source_table(Grid *g)
 }
 
 // deinterleave AoS float (stride s) into up to 6 SoA arrays; per component c
-// flag[c] bit 1 = some value differs from `ref`, bit 2 = some value is not finite
+// flag[c] bit 1 = some value differs from `ref`, bit 2 = some value is not finite,
+// bit 4 (c = 1, 2) = some cell's value differs from its component 0
 __global__ void k_deinterleave(const float *aos, int stride, float *d0, float *d1, float *d2, float *d3, float *d4,
                                float *d5, long long n, float ref, int *flag)
 {
     float *d[6] = {d0, d1, d2, d3, d4, d5};
     int local[6] = {0, 0, 0, 0, 0, 0};
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const float v0 = aos[q * stride];
 #pragma unroll
         for (int c = 0; c < 6; c++) {
             if (c >= stride) break;
@@ -436,6 +440,7 @@ __global__ void k_deinterleave(const float *aos, int stride, float *d0, float *d
             d[c][q] = v;
             if (v != ref) local[c] |= 1;
             if (!isfinite(v)) local[c] |= 2;
+            if ((c == 1 || c == 2) && v != v0) local[c] |= 4;
         }
     }
     for (int c = 0; c < stride; c++)
@@ -495,6 +500,7 @@ bool grid_upload_materials(Grid *g)
     g->mu_nonunit = ((g->h_flag[3] | g->h_flag[4] | g->h_flag[5]) & 1) != 0;
     g->sig_e = ((g->h_flag[6] | g->h_flag[7] | g->h_flag[8]) & 1) != 0;
     g->sig_m = ((g->h_flag[9] | g->h_flag[10] | g->h_flag[11]) & 1) != 0;
+    g->mat_iso = ((g->h_flag[1] | g->h_flag[2] | g->h_flag[7] | g->h_flag[8]) & 4) == 0;
     g->mat_dirty = 0;
     g->coef_valid = false;
     g->version++;
@@ -671,13 +677,22 @@ static bool fast32_path(const Grid *g)
     return g->prec == FDTD_F32 && g->boundary != FDTD_BOUNDARY_MUR && !g->sig_m && !g->mu_nonunit;
 }
 
-// which kernel design the fast path uses: the one-pass streaming kernel where
-// the grid allows it (FDTD_YEE_STREAM, and FDTD_YEE_AUTO: it moves each array
-// once a step and measured faster than the flat pair with and without CPML),
-// the plane-streaming TMA / cp.async kernel on request, else the flat pair
+// which kernel design the fast path uses: the one-pass streaming step where the
+// grid allows it (FDTD_YEE_STREAM, and FDTD_YEE_AUTO: it moves each array once a
+// step and measured faster than the flat pair with and without CPML), the
+// plane-streaming TMA / cp.async kernel on request, else the flat pair.  The
+// streaming step has two kernels: with one E coefficient a cell (yee_tile.cu, 52
+// B a cell, tiles that may split the rows) where a cell's three agree, else with
+// three (yee_stream.cu, 60 B).
+static bool tile_path(const Grid *g)
+{
+    return fast32_path(g) && (g->yee_variant == FDTD_YEE_STREAM || g->yee_variant == FDTD_YEE_AUTO) && g->mat_iso &&
+           tile_supported(g->nx, g->ny, g->nz, g->sig_e, g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0);
+}
+
 static bool stream_path(const Grid *g)
 {
-    return fast32_path(g) && (g->yee_variant == FDTD_YEE_STREAM || g->yee_variant == FDTD_YEE_AUTO) &&
+    return fast32_path(g) && (g->yee_variant == FDTD_YEE_STREAM || g->yee_variant == FDTD_YEE_AUTO) && !tile_path(g) &&
            stream_supported(g->nx, g->ny, g->nz, g->sig_e, g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0);
 }
 
@@ -687,7 +702,7 @@ static bool fused_path(const Grid *g)
 }
 
 // designs that read one field set and write the other
-static bool pingpong_path(const Grid *g) { return stream_path(g) || fused_path(g); }
+static bool pingpong_path(const Grid *g) { return tile_path(g) || stream_path(g) || fused_path(g); }
 
 // tile plan of the streaming kernel for the grid's shape (rebuilt when the
 // shape, CPML thickness, loss or device changes)
@@ -715,6 +730,49 @@ static bool stream_prepare(Grid *g)
     CK(cudaMemcpyAsync(g->d_tiles, p.tiles.data(), p.tiles.size() * sizeof(StreamTile), cudaMemcpyHostToDevice, g->st));
     g->splan = std::move(p);
     std::copy(key, key + 6, g->splan_key);
+    g->version++;
+    return true;
+}
+
+// the same for the one-coefficient kernel
+static bool tile_prepare(Grid *g)
+{
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int L = g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0;
+    const int key[6] = {g->nx, g->ny, g->nz, L, g->sig_e ? 1 : 0, nsm};
+    const void *arrays[14] = {g->cb[0], g->sig_e ? g->ca[0] : nullptr};
+    for (int s = 0; s < 2; s++)
+        for (int m = 0; m < 6; m++) arrays[2 + 6 * s + m] = g->f[s][m];
+    const bool same_plan = g->d_boxes && std::equal(key, key + 6, g->tplan_key);
+    if (same_plan && std::equal(arrays, arrays + 14, g->maps_of)) return true;
+    TilePlan p;
+    if (!tile_plan(g->nx, g->ny, g->nz, L, g->sig_e, nsm, &p)) {
+        set_error(FDTD_ERR_UNSUPPORTED, "streaming Yee kernel: no tile plan for grid %dx%dx%d", g->nx, g->ny, g->nz);
+        return false;
+    }
+    if (!tile_configure(p.smem, p.threads)) {
+        set_error(FDTD_ERR_CUDA, "streaming Yee kernel: blocks of %d threads with %zu bytes of shared memory cannot launch",
+                  p.threads, p.smem);
+        return false;
+    }
+    CK(cudaStreamSynchronize(g->st));
+    dfree(g->d_boxes);
+    if (!dalloc(&g->d_boxes, p.tiles.size() * sizeof(TileBox), g->st, false)) return false;
+    CK(cudaMemcpyAsync(g->d_boxes, p.tiles.data(), p.tiles.size() * sizeof(TileBox), cudaMemcpyHostToDevice, g->st));
+    TileMaps maps[2];
+    for (int s = 0; s < 2; s++)
+        if (!tile_make_maps(&maps[s], (const float *const *)g->f[s], g->cb[0], g->sig_e ? g->ca[0] : nullptr, g->nx,
+                            g->ny, g->nz, p)) {
+            set_error(FDTD_ERR_CUDA, "streaming Yee kernel: TMA descriptors of a %dx%dx%d grid", g->nx, g->ny, g->nz);
+            return false;
+        }
+    if (!dalloc(&g->d_maps, sizeof maps, g->st, false)) return false;
+    CK(cudaMemcpyAsync(g->d_maps, maps, sizeof maps, cudaMemcpyHostToDevice, g->st));
+    g->tplan = std::move(p);
+    std::copy(key, key + 6, g->tplan_key);
+    std::copy(arrays, arrays + 14, g->maps_of);
     g->version++;
     return true;
 }
@@ -801,6 +859,7 @@ bool grid_prepare_step(Grid *g, double dt)
             g->fmaps[0] = g->fmaps[1] = nullptr;
             g->version++;
         }
+        if (tile_path(g) && !tile_prepare(g)) return false;
         if (stream_path(g) && !stream_prepare(g)) return false;
         // TMA descriptors of the fused kernel (host-side encode; they only depend on the buffers)
         if (fused_path(g) && !g->fmaps[0] && fused_tma_supported(g->nx, g->ny, g->nz)) {
@@ -981,13 +1040,13 @@ static bool step_fused(Grid *g, double dt)
     return true;
 }
 
-static bool step_stream(Grid *g, double dt)
+// the streaming step's arguments with field set `in` as input
+static StreamArgs stream_args(Grid *g, int in, double dt)
 {
     StreamArgs a{};
     a.nx = g->nx; a.ny = g->ny; a.nz = g->nz;
     a.L = g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0;
-    a.ty = g->splan.ty;
-    const int in = g->cur, out = 1 - g->cur;
+    const int out = 1 - in;
     for (int m = 0; m < 6; m++) { a.f_in[m] = (const float *)g->f[in][m]; a.f_out[m] = (float *)g->f[out][m]; }
     for (int c = 0; c < 3; c++) { a.cb[c] = g->cb[c]; a.ca[c] = g->sig_e ? g->ca[c] : nullptr; }
     a.hb = (float)(dt / g->dx);
@@ -1000,10 +1059,21 @@ static bool step_stream(Grid *g, double dt)
         for (int w = 0; w < 6; w++) a.prof[w][ax] = (const float *)g->prof[w][ax];
     }
     a.src = source_table(g);
-    a.tiles = g->d_tiles;
-    launch_yee_stream(a, g->splan, g->st);
+    return a;
+}
+
+static bool step_stream(Grid *g, double dt)
+{
+    StreamArgs a = stream_args(g, g->cur, dt);
+    if (tile_path(g)) {
+        launch_yee_tile(a, g->d_maps + g->cur, g->d_boxes, g->tplan, g->d_err, g->st);
+    } else {
+        a.ty = g->splan.ty;
+        a.tiles = g->d_tiles;
+        launch_yee_stream(a, g->splan, g->st);
+    }
     CKL("streaming step");
-    g->cur = out;
+    g->cur = 1 - g->cur;
     return true;
 }
 
@@ -1128,7 +1198,7 @@ bool enqueue_step(Grid *g, double dt, bool with_extras)
     // read after a replay (a plain record during capture is only a dependency)
     if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step], g->st, cudaEventRecordExternal));
     if (g->prec == FDTD_F64) ok = step_split<double>(g, dt, with_extras);
-    else if (stream_path(g)) ok = step_stream(g, dt);
+    else if (tile_path(g) || stream_path(g)) ok = step_stream(g, dt);
     else if (fused_path(g)) ok = step_fused(g, dt);
     else if (fast32_path(g)) ok = step_flat(g, dt);
     else ok = step_split<float>(g, dt, with_extras);
@@ -1348,8 +1418,12 @@ bool drain_kernel_timing(Grid *g, int set)
 static bool run_steps_in(Grid *g, double dt, int nsteps);
 
 // ============================================================================
-// candidate sweeps: many grids in persistent launches (yee_sweep.cu)
+// candidate sweeps: many grids at once (the one-coefficient kernel on the grids'
+// own streams; the others in persistent launches, yee_sweep.cu)
 // ============================================================================
+static bool run_sweep_persistent(const std::vector<Grid *> &gs, double dt, const std::vector<int> &nsteps,
+                                 int steps_per_launch, int ty_cap, double tiles_per_sm);
+
 bool run_sweep(const std::vector<Grid *> &gs, double dt, const std::vector<int> &nsteps, int steps_per_launch,
                int ty_cap, double tiles_per_sm)
 {
@@ -1383,15 +1457,52 @@ bool run_sweep(const std::vector<Grid *> &gs, double dt, const std::vector<int> 
         }
     }
     // every grid on the one-pass path (two field and auxiliary sets), prepared
-    // as for timefield3d_run; the first step's scheduled source written
-    cudaStream_t sst = sweep_stream();
-    for (Grid *g : gs) {
+    // as for timefield3d_run
+    std::vector<Grid *> rest;
+    std::vector<int> rest_steps;
+    std::vector<std::pair<Grid *, int>> alone;
+    for (int i = 0; i < ng; i++) {
+        Grid *g = gs[i];
         if (g->yee_variant != FDTD_YEE_STREAM) {
             g->yee_variant = FDTD_YEE_STREAM;
             g->pp_synced = false;
             g->version++;
         }
         if (!prepare_run(g, dt)) return false;
+        if (tile_path(g)) {
+            alone.push_back({g, nsteps[i]});
+        } else {
+            rest.push_back(g);
+            rest_steps.push_back(nsteps[i]);
+        }
+    }
+    // Grids with one E coefficient a cell run as timefield3d_run would, each on its
+    // own stream: a step's tiles fill the device, and where one grid's last tiles
+    // leave SMs idle another's blocks start.  Eight candidates of 256x128 cells, 160
+    // steps: 113 ms, against 192 in the persistent launches, whose tiles carry three
+    // coefficients and whose steps meet at two grid barriers.
+    for (auto &[g, n] : alone) {
+        const int ktime = g->ktime;
+        g->ktime = 0;
+        const bool ok = run_steps(g, dt, n);
+        g->ktime = ktime;
+        if (!ok) return false;
+    }
+    return rest.empty() || run_sweep_persistent(rest, dt, rest_steps, steps_per_launch, ty_cap, tiles_per_sm);
+}
+
+// grids checked and prepared by run_sweep
+static bool run_sweep_persistent(const std::vector<Grid *> &gs, double dt, const std::vector<int> &nsteps,
+                                 int steps_per_launch, int ty_cap, double tiles_per_sm)
+{
+    const int ng = (int)gs.size();
+    int nsm = 0;
+    if (!sweep_setup(&nsm)) return false;
+    const Grid *g0 = gs[0];
+    const int L0 = g0->boundary == FDTD_BOUNDARY_CPML ? g0->L : 0;
+    // the first step's scheduled source
+    cudaStream_t sst = sweep_stream();
+    for (Grid *g : gs) {
         if (g->sched.active && !enqueue_schedule(g, 0)) return false;
         CK(cudaEventRecord(g->ev_fork, g->st));
         CK(cudaStreamWaitEvent(sst, g->ev_fork, 0));

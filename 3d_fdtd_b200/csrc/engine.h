@@ -127,6 +127,13 @@ struct Grid {
     StreamPlan splan;
     StreamTile *d_tiles = nullptr;
     int splan_key[6] = {-1, -1, -1, -1, -1, -1};   // nx ny nz L lossy nsm the plan was built for
+    // the same step where every cell's three E coefficients agree (yee_tile.cu)
+    TilePlan tplan;
+    TileBox *d_boxes = nullptr;
+    TileMaps *d_maps = nullptr;      // two: set 0, set 1 as input
+    const void *maps_of[14] = {};    // the arrays they describe
+    int tplan_key[6] = {-1, -1, -1, -1, -1, -1};
+    bool mat_iso = false;            // ep and electric sig equal on a cell's three components, every cell
     int *d_err = nullptr;            // device error flag (a bounded wait gave up)
     int *h_err = nullptr;            // pinned
 

@@ -236,6 +236,35 @@ double stream_tile_cost(int nx, int ny, int nz, int L, const StreamTile &t);
 bool stream_configure(size_t smem, int threads);
 void launch_yee_stream(const StreamArgs &a, const StreamPlan &p, cudaStream_t st);
 
+// yee_tile.cu: the same one-pass step where the three E coefficients of every
+// cell are equal (cb[0], ca[0] only), in tiles that may also split the rows
+struct TileBox {
+    int q0, q1;              // owned quads (4 x cells) [q0, q1)
+    int j0, rows;            // owned rows
+    int k0, k1;              // owned planes
+};
+struct TilePlan {
+    int tp = 0, sw = 0;          // staged rows, slots a row of a block's shared memory
+    int threads = 0;
+    size_t smem = 0;             // bytes
+    std::vector<TileBox> tiles;  // a block each, in the order they start
+    double span = 0;             // estimate of the launch (us)
+};
+int tile_supported(int nx, int ny, int nz, bool lossy, int L);
+// tiles for a grid over nsm blocks; ty_cap > 0 caps the rows of a band
+bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out, int ty_cap = 0);
+bool tile_configure(size_t smem, int threads);
+// TMA descriptors of one input set, in device memory
+struct TileMaps {
+    CUtensorMap h[3];        // boxes of sw quads x (tp + 1) rows
+    CUtensorMap e[3];        // x tp rows
+    CUtensorMap cb, ca;      // ca: unused without loss
+};
+bool tile_make_maps(TileMaps *m, const float *const f[6], const float *cb, const float *ca, int nx, int ny, int nz,
+                    const TilePlan &p);
+// err: device flag set when a bounded wait gave up
+void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *tiles, const TilePlan &p, int *err, cudaStream_t st);
+
 // yee_sweep.cu: many grids advanced together by persistent launches of S
 // steps (see the file's header); one entry per grid per launch
 constexpr int kSweepMaxGrids = 48;   // grids of one sweep call (their tile arguments sit in constant memory)
@@ -331,6 +360,8 @@ struct FusedMaps {
     CUtensorMap ca[3];
 };
 int fused_tma_supported(int nx, int ny, int nz);
+// descriptor of an nx x ny x nz float array, boxes of box_x x box_y cells of one plane
+bool tma_encode_3d(CUtensorMap *m, const float *base, int nx, int ny, int nz, int box_x, int box_y);
 bool fused_make_maps(FusedMaps *m, const float *const f[6], const float *const cb[3], const float *const ca[3],
                      int nx, int ny, int nz);
 void launch_fused_step_tma(const FusedArgs &a, const FusedMaps &m, int *err, cudaStream_t st);

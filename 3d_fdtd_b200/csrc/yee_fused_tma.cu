@@ -530,8 +530,9 @@ constexpr int kTY = 8;   // tile height (rows per thread = kTY / 8)
 
 int fused_tma_supported(int nx, int ny, int nz) { return nx % 4 == 0 && nx >= 8 && ny >= 4 && nz >= 4 && encode_fn(); }
 
-static bool encode(CUtensorMap *m, const float *base, int nx, int ny, int nz, int box_x, int box_y)
+bool tma_encode_3d(CUtensorMap *m, const float *base, int nx, int ny, int nz, int box_x, int box_y)
 {
+    if (!encode_fn()) return false;
     cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
     cuuint64_t strides[2] = {(cuuint64_t)nx * 4, (cuuint64_t)nx * ny * 4};
     cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1};
@@ -547,11 +548,11 @@ bool fused_make_maps(FusedMaps *m, const float *const f[6], const float *const c
 {
     if (!encode_fn()) return false;
     for (int c = 0; c < 3; c++) {
-        if (!encode(&m->h[c], f[3 + c], nx, ny, nz, HW, kTY + 2)) return false;
-        if (!encode(&m->e[c], f[c], nx, ny, nz, EW, kTY + 1)) return false;
-        if (!encode(&m->cb[c], cb[c], nx, ny, nz, EW, kTY + 1)) return false;
+        if (!tma_encode_3d(&m->h[c], f[3 + c], nx, ny, nz, HW, kTY + 2)) return false;
+        if (!tma_encode_3d(&m->e[c], f[c], nx, ny, nz, EW, kTY + 1)) return false;
+        if (!tma_encode_3d(&m->cb[c], cb[c], nx, ny, nz, EW, kTY + 1)) return false;
         if (ca && ca[c]) {
-            if (!encode(&m->ca[c], ca[c], nx, ny, nz, EW, kTY + 1)) return false;
+            if (!tma_encode_3d(&m->ca[c], ca[c], nx, ny, nz, EW, kTY + 1)) return false;
         } else {
             m->ca[c] = m->cb[c];
         }

@@ -465,15 +465,17 @@ void fdtd_inject_allocation_failures(int n);
  * the CUDA context still usable; *elapsed_seconds = the device-side wait. */
 int fdtd_wait_selftest(double limit_seconds, double *elapsed_seconds);
 /* Candidate sweep: advance `ngrids` grids together, grid i by nsteps[i] steps
- * (uneven counts allowed), in persistent launches of up to steps_per_launch
- * steps that run every grid's one-pass Yee update, monitors and scheduled
- * source (captured as one CUDA graph on the library's sweep stream; returns
- * at once, each grid's stream continues after it).  No reference counterpart:
- * the reference runs one design at a time (3d_fdtd.c:93-202).  Each grid is
- * set up as for timefield3d_run (FP32, CPML of the same thickness on all or
- * PEC walls on all, the same loss, nx a multiple of 4, no probes or bound
- * stores) and ends exactly as timefield3d_run would leave it.  Tile shape:
- * band_rows caps the rows of a band (0: as many as shared memory allows);
+ * (uneven counts allowed); returns at once, each grid's stream continues after
+ * it.  No reference counterpart: the reference runs one design at a time
+ * (3d_fdtd.c:93-202).  Each grid is set up as for timefield3d_run (FP32, CPML of
+ * the same thickness on all or PEC walls on all, the same loss, nx a multiple
+ * of 4, no probes or bound stores) and ends exactly as timefield3d_run would
+ * leave it.  Grids whose permittivity and conductivity agree on the three
+ * components of every cell are enqueued on their own streams and share the
+ * device; the arguments below are for the others, which run in persistent
+ * launches of up to steps_per_launch steps (every grid's Yee update, monitors
+ * and scheduled source, captured as one CUDA graph on the library's sweep
+ * stream).  Tile shape: band_rows caps the rows of a band (0: as many as shared memory allows);
  * tiles_per_sm sets how many tiles per SM the grids are cut into per step
  * (in (0, 16]; the blocks take the tiles of all grids from one queue, longest
  * first, so finer tiles balance better).  At most 48 grids per call.  A grid barrier that waits more than 1 s ends the launch;
