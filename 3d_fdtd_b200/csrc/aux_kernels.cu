@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) k_step_tail(TailArgs a)
         const OverlapJob jb = a.jobs[jid];
         overlap_block<T>((const T *const *)a.f, a.nx, a.ny, jb, part, a.nparts, a.partials + b);
     } else {
-        const SrcStep v = schedule_step(a.src, *a.step + 1);
+        const SrcStep v = schedule_step(a.src, *a.step + a.offset + 1);
         mode_source_cells(a.src, (b - nov) * (long long)blockDim.x + threadIdx.x,
                           (long long)a.src_blocks * blockDim.x, v);
     }
@@ -127,7 +127,11 @@ __global__ void __launch_bounds__(256) k_step_tail(TailArgs a)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const long long n = *a.step;
+    const long long n = *a.step + a.offset;
+    if (a.prev) {
+        chain_add_up(a.jobs, a.njobs, a.nparts, a.prev, a.scale, a.dt, n - 1, threadIdx.x >> 5, blockDim.x >> 5);
+        __syncthreads();
+    }
     // stage every partial in shared memory, then one thread per job adds its
     // partials in order (the order of k_overlap_finalize)
     constexpr int kStage = 1024;
@@ -215,7 +219,7 @@ __global__ void k_probes(const T *const *f, const ProbeJob *probes, int np, doub
     count[p] = c + 1;
 }
 
-__global__ void k_step_advance(long long *step) { *step += 1; }
+__global__ void k_step_advance(long long *step, int by) { *step += by; }
 
 // ---------------------------------------------------------------------------
 // Taper edge store (adjoint3d.c:259-337): gather E (3 components) at the
@@ -343,7 +347,7 @@ void launch_step_tail(TailArgs a, cudaStream_t st)
     const int blocks = a.njobs * a.nparts + a.src_blocks;
     note_launch();
     if (blocks == 0) {
-        k_step_advance<<<1, 1, 0, st>>>(a.step);
+        k_step_advance<<<1, 1, 0, st>>>(a.step, a.offset + 1);
         return;
     }
     // launched with a programmatic dependency on the preceding kernel (see k_step_tail)
@@ -420,7 +424,7 @@ void launch_probes(const T *const *f_dev, const ProbeJob *probes, int np, double
 void launch_step_advance(long long *step, cudaStream_t st)
 {
     note_launch();
-    k_step_advance<<<1, 1, 0, st>>>(step);
+    k_step_advance<<<1, 1, 0, st>>>(step, 1);
 }
 
 template <typename T>

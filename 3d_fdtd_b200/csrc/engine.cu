@@ -376,6 +376,8 @@ Grid::~Grid()
         dfree(d_tiles);
         dfree(d_boxes);
         dfree(d_maps);
+        dfree(d_sums);
+        dfree(d_src2);
         dfree(d_flag);
         for (auto &mn : monitors) { dfree(mn.d_omega); dfree(mn.d_acc); priv_mode_free(mn.mode_key); }
         dfree(d_probes); dfree(d_probe_buf); dfree(d_probe_count);
@@ -1066,7 +1068,7 @@ static bool step_stream(Grid *g, double dt)
 {
     StreamArgs a = stream_args(g, g->cur, dt);
     if (tile_path(g)) {
-        launch_yee_tile(a, g->d_maps + g->cur, g->d_boxes, g->tplan, g->d_err, g->st);
+        launch_yee_tile(a, g->d_maps + g->cur, g->d_boxes, g->tplan, StepChain{}, g->d_err, g->st);
     } else {
         a.ty = g->splan.ty;
         a.tiles = g->d_tiles;
@@ -1205,6 +1207,113 @@ bool enqueue_step(Grid *g, double dt, bool with_extras)
     if (!ok) return false;
     if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step + 1], g->st, cudaEventRecordExternal));
     return with_extras ? enqueue_after_step(g, dt) : true;
+}
+
+// ============================================================================
+// chains of steps (StepChain): the one-coefficient kernel's graphs
+// ============================================================================
+// probes keep their order with the step's other launches
+static bool chain_path(const Grid *g)
+{
+    return tile_path(g) && g->probes.empty() && g->binds.size() <= (size_t)kChainStores;
+}
+
+// scratch of a chain, and the source plane of its odd steps as the user left it
+// (cells outside the mode's window keep their values)
+static bool chain_prepare(Grid *g)
+{
+    const size_t sums = 2 * (size_t)g->njobs * (g->njobs ? overlap_parts(g->job_cells) : 0) * 8 * sizeof(double2);
+    if (g->sums_cap < sums) {
+        CK(cudaStreamSynchronize(g->st));
+        dfree(g->d_sums);
+        g->sums_cap = 0;
+        if (!dalloc(&g->d_sums, sums, g->st, false)) return false;
+        g->sums_cap = sums;
+        g->version++;
+    }
+    if (!g->sched.active) return true;
+    const size_t bytes = 6 * (size_t)g->nx * g->ny * sizeof(float);
+    if (!g->d_src2) {
+        if (!dalloc(&g->d_src2, bytes, g->st, false)) return false;
+        g->version++;
+    }
+    Plane *pl = grid_plane(g, g->sched.cz, false);
+    if (!pl) {
+        set_error(FDTD_ERR_ARG, "scheduled source not prepared");
+        return false;
+    }
+    CK(cudaMemcpyAsync(g->d_src2, pl->p, bytes, cudaMemcpyDeviceToDevice, g->st));
+    return true;
+}
+
+// step s of a chain of n: the tiles, the end of step s - 1 and the sums of step
+// s - 2; after the last one its own end
+static bool enqueue_chain_step(Grid *g, double dt, int s, int n)
+{
+    StreamArgs a = stream_args(g, g->cur, dt);
+    StepChain c{};
+    c.f = (const float *const *)g->d_fptr[g->cur];
+    c.jobs = g->d_jobs;
+    c.njobs = g->njobs;
+    c.nparts = g->njobs ? overlap_parts(g->job_cells) : 0;
+    c.scale = -0.5 * g->dx * g->dx;
+    c.dt = dt;
+    c.step = g->d_step;
+    c.s = s;
+    const size_t half = (size_t)g->njobs * c.nparts * 8;
+    if (g->njobs && s >= 1) c.sums = g->d_sums + (s & 1) * half;
+    if (g->njobs && s >= 2) c.prev = g->d_sums + (1 - (s & 1)) * half;
+    c.units = c.sums ? (int)half : 0;
+    if (g->sched.active) {
+        Plane *pl = grid_plane(g, g->sched.cz, false);
+        for (int i = 0; pl && i < a.src.n; i++)
+            if (a.src.p[i] == pl->p && (s & 1)) a.src.p[i] = g->d_src2;
+        if (s + 1 < n) {
+            if (!schedule_job(g, &c.src)) return false;
+            if (!(s & 1)) c.src.plane = g->d_src2;
+            c.src.win = mode_window(c.src.nx, c.src.ny, c.src.cx, c.src.cy, c.src.mi, c.src.mj, c.src.ratio);
+            c.src_units = (int)std::min<long long>(((long long)c.src.win.wni * c.src.win.wnj + 31) / 32, 1 << 20);
+            c.units += c.src_units;
+        }
+    }
+    if (s >= 1)
+        for (auto &b : g->binds) {
+            adjoint3d_taper key{};
+            key.left = (int *)b.taper_key;
+            TaperDev *td = taper_lookup(key, false);
+            if (!td) continue;
+            c.store[c.nstores++] = ChainStore{td->d_cells, (float *)(b.which ? td->d_adj : td->d_fwd), td->ncell, b.t0,
+                                              b.dir, td->duration};
+            c.units += (td->ncell + 31) / 32;
+        }
+    c.blocks = std::min((int)g->tplan.tiles.size(), g->tplan_key[5]);
+    if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step], g->st, cudaEventRecordExternal));
+    launch_yee_tile(a, g->d_maps + g->cur, g->d_boxes, g->tplan, c, g->d_err, g->st);
+    if (g->cap_ev) CK(cudaEventRecordWithFlags(g->cap_ev[2 * g->cap_step + 1], g->st, cudaEventRecordExternal));
+    CKL("streaming step");
+    g->cur = 1 - g->cur;
+    if (s + 1 < n) return true;
+    for (auto &b : g->binds) {
+        adjoint3d_taper key{};
+        key.left = (int *)b.taper_key;
+        TaperDev *td = taper_lookup(key, false);
+        if (td && !enqueue_taper_store(td, g, b.which, 0, g->d_step, b.t0 + b.dir * s, b.dir)) return false;
+    }
+    TailArgs t{};
+    t.f = (const void *const *)g->d_fptr[g->cur];
+    t.nx = g->nx; t.ny = g->ny;
+    t.jobs = g->d_jobs; t.njobs = g->njobs;
+    t.cells = g->job_cells;
+    t.partials = g->d_partials;
+    t.scale = c.scale; t.dt = dt;
+    t.step = g->d_step;
+    t.done = g->d_done;
+    t.offset = s;
+    if (c.sums) t.prev = c.sums;
+    if (g->sched.active && !schedule_job(g, &t.src)) return false;
+    launch_step_tail<float>(t, g->st);
+    CKL("after step");
+    return true;
 }
 
 // ============================================================================
@@ -1357,13 +1466,14 @@ static bool capture_graph(Grid *g, int slot, double dt)
         g->cap_ev = g->kev[slot - 1];
     }
     const int cur0 = g->cur;
+    const bool chain = chain_path(g);
     const long long before = launch_count();
     cudaGraph_t gr;
     CK(cudaStreamBeginCapture(g->st, cudaStreamCaptureModeThreadLocal));
     bool ok = true;
     for (int s = 0; s < kGraphSteps && ok; s++) {
         g->cap_step = s;
-        ok = enqueue_step(g, dt, true);
+        ok = chain ? enqueue_chain_step(g, dt, s, kGraphSteps) : enqueue_step(g, dt, true);
     }
     g->cap_ev = nullptr;
     cudaError_t ce = cudaStreamEndCapture(g->st, &gr);
@@ -1656,6 +1766,7 @@ static bool run_steps_in(Grid *g, double dt, int nsteps)
         return true;
     }
     int full = nsteps / kGraphSteps, rest = nsteps % kGraphSteps;
+    if (full > 0 && chain_path(g) && !chain_prepare(g)) return false;
     if (full > 0 && !g->ktime) {
         if (!capture_graph(g, 0, dt)) return false;
         for (int r = 0; r < full; r++) {

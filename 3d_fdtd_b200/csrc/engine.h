@@ -133,6 +133,9 @@ struct Grid {
     TileMaps *d_maps = nullptr;      // two: set 0, set 1 as input
     const void *maps_of[14] = {};    // the arrays they describe
     int tplan_key[6] = {-1, -1, -1, -1, -1, -1};
+    double2 *d_sums = nullptr;       // a chain's overlap sums, two steps (StepChain)
+    size_t sums_cap = 0;
+    float *d_src2 = nullptr;         // the scheduled source's plane on odd steps of a chain
     bool mat_iso = false;            // ep and electric sig equal on a cell's three components, every cell
     int *d_err = nullptr;            // device error flag (a bounded wait gave up)
     int *h_err = nullptr;            // pinned

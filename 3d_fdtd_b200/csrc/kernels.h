@@ -99,6 +99,41 @@ struct TailArgs {
     SourceJob src;
     int src_blocks;
     unsigned *done;             // completion count, 0 between launches
+    int offset;                 // the step is *step + offset (a chain's last one, see StepChain)
+    const double2 *prev;        // a chain's overlap sums of the step before it (null: none)
+};
+
+// A chain of steps in which a step's launch takes along the end of the step before
+// it (yee_tile.cu): its overlaps and edge stores from the fields that are this
+// launch's input, as units of one warp each, and the next step's source plane.  The
+// overlap sums are added up one launch later.  Nothing but the next-but-one launch
+// waits for any of it.  The step counter stands still until the chain's end.  A tail
+// launch between two steps is latency that nothing hides (a block of the step takes a
+// whole SM, so none of the tail's starts beside one): a step with two monitors of 11
+// frequencies and a source took 175 us on 200x160x400, 164.7 in a chain, 160 without
+// them; one with edge stores on 256x128x128 81 us, 73 in a chain.
+constexpr int kChainStores = 4;
+struct ChainStore {
+    const long long *cells;
+    float *store;
+    int ncell, t0, dir, duration;   // as launch_taper_store
+};
+struct StepChain {
+    const float *const *f;      // device array of the input's six field pointers
+    const OverlapJob *jobs;
+    int njobs, nparts;
+    double2 *sums;              // the previous step's warp sums, [job][part][8] (null: none)
+    const double2 *prev;        // those of the step before it, to be added up (null: none)
+    double scale, dt;
+    const long long *step;      // steps taken when the chain starts
+    int s;                      // this step of the chain
+    SourceJob src;              // the next step's source (plane null: none)
+    int src_units;
+    int nstores;
+    ChainStore store[kChainStores];
+    int units;                  // in all, shared by the first `blocks` blocks
+    int blocks;
+    int ntiles;                 // block ntiles adds up `prev`
 };
 
 struct ProbeJob {
@@ -263,7 +298,8 @@ struct TileMaps {
 bool tile_make_maps(TileMaps *m, const float *const f[6], const float *cb, const float *ca, int nx, int ny, int nz,
                     const TilePlan &p);
 // err: device flag set when a bounded wait gave up
-void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *tiles, const TilePlan &p, int *err, cudaStream_t st);
+void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *tiles, const TilePlan &p, StepChain chain,
+                     int *err, cudaStream_t st);
 
 // yee_sweep.cu: many grids advanced together by persistent launches of S
 // steps (see the file's header); one entry per grid per launch
@@ -375,7 +411,7 @@ void launch_mode_source(float *plane, const float *const ep_plane[3], const floa
 void launch_mode_source_job(const SourceJob &sj, double amplitude, double cph, double sph, const long long *step,
                             int step_offset, cudaStream_t st);
 template <typename T>
-void launch_step_tail(TailArgs a, cudaStream_t st);
+void launch_step_tail(TailArgs a, cudaStream_t st);   // nparts, src.win, src_blocks are set here
 void launch_set_value(float *p, long long idx, float v, cudaStream_t st);
 int overlap_parts(long long cells);
 // cells: the largest overlap window (win.wni * win.wnj) of the jobs

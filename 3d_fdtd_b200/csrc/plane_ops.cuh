@@ -271,4 +271,41 @@ __device__ __forceinline__ void accumulate_frequency(const OverlapJob &jb, int f
     jb.acc[2 * f + 1] = comp;
 }
 
+// Eight warp sums of every partial (overlap_block's, kept apart) of every job, added
+// up and accumulated as the step tail does, one warp a job (all threads call it; nw
+// warps).  Four partials at a time: lanes 8q + v hold warp sum v of partial q, so the
+// block's last reduction, whose other lanes hold 0, is the same additions.
+__device__ __forceinline__ void chain_add_up(const OverlapJob *jobs, int njobs, int nparts, const double2 *sums,
+                                             double scale, double dt, long long n, int warp, int nw)
+{
+    const int lane = threadIdx.x & 31;
+    for (int jid = warp; jid < njobs; jid += nw) {
+        const OverlapJob jb = jobs[jid];
+        const double2 *s = sums + (size_t)jid * nparts * 8;
+        double sre = 0.0, sim = 0.0;
+        for (int p = 0; p < nparts; p += 4) {
+            const int u = p * 8 + lane;
+            double2 v = u < nparts * 8 ? __ldcg(s + u) : make_double2(0.0, 0.0);
+            v.x = dadd(v.x, 0.0);
+            v.y = dadd(v.y, 0.0);
+            for (int o = 4; o > 0; o >>= 1) {
+                v.x = dadd(v.x, __shfl_down_sync(0xffffffffu, v.x, o, 8));
+                v.y = dadd(v.y, __shfl_down_sync(0xffffffffu, v.y, o, 8));
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const double x = __shfl_sync(0xffffffffu, v.x, 8 * q), y = __shfl_sync(0xffffffffu, v.y, 8 * q);
+                if (p + q < nparts) {
+                    sre = dadd(sre, x);
+                    sim = dadd(sim, y);
+                }
+            }
+        }
+        const double2 tot = make_double2(dmul(scale, sre), dmul(scale, sim));
+        if (jb.inst && lane == 0) *jb.inst = tot;
+        if (jb.acc)
+            for (int f = lane; f < jb.nfreq; f += 32) accumulate_frequency(jb, f, tot, dt, n);
+    }
+}
+
 }  // namespace fdtd

@@ -139,9 +139,13 @@ __device__ __forceinline__ void tile_box(float *dst, const CUtensorMap *map, int
 // the auxiliaries of the next plane, loaded an iteration ahead, need the
 // registers.  The two kinds of planes are loops of their own, so neither holds
 // the other's state.
-template <bool CPML, bool LOSSY>
+//
+// before(): run by all threads before the copies of the first planes; during(): while
+// they are on their way.
+template <bool CPML, bool LOSSY, typename Before, typename During>
 __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox tl,
-                                         const TileShape sh, float *sm, TileSync *sync, int *err)
+                                         const TileShape sh, float *sm, TileSync *sync, int *err, Before before,
+                                         During during)
 {
     constexpr int S = kStreamStages;
     const int nx = a.nx, ny = a.ny, nz = a.nz, L = CPML ? a.L : 0;
@@ -161,9 +165,8 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
     float *xps = enew + 2 * M::kENew;                    // [S][4][TP][XW]
     float *ptab = xps + S * xp_st;
     if (CPML) stream_profile_table(ptab, a);
-    __syncthreads();
     const int NT = ro.threads;
-    if (tid >= NT) return;
+    before();
     // thread 0 copies: one TMA box a plane and array.  Plane it + 2 goes into the
     // stage of plane it - 1 right after the barrier of iteration it, when every
     // thread is done with iteration it - 1.
@@ -189,6 +192,9 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
         copy(0, false);
         copy(1, false);      // a tile has at least one plane
     }
+    during();
+    __syncthreads();
+    if (tid >= NT) return;
     auto wait_plane = [&](int it) {
         const int m = it + 1;
         tile_wait(sync, &sync->full[m % S], (unsigned)(m / S) & 1u);

@@ -23,6 +23,7 @@
 // CPML 792 and 415; 256x128x128 CPML 77 and 67; 96x80x64 CPML, conductivity 45 and
 // 14.5 us.  Two blocks an SM (96 registers) spill with CPML and gave nothing without.
 #include "tile_cells.cuh"
+#include "plane_ops.cuh"
 
 #include <algorithm>
 
@@ -31,20 +32,65 @@ namespace fdtd {
 constexpr int kTileMaxThreads = 512;
 constexpr size_t kTileSmemBudget = kStreamSmemBudget;
 
+// the units of a chain (StepChain), unit u by warp u / blocks of block u % blocks
+__device__ __forceinline__ void chain_units(const StepChain &c, int nx, int ny)
+{
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int nov = c.sums ? c.njobs * c.nparts * 8 : 0;
+    for (int u = (threadIdx.x >> 5) * c.blocks + blockIdx.x; u < c.units; u += nw * c.blocks) {
+        if (u < nov) {
+            const int part = (u >> 3) % c.nparts;
+            const OverlapJob jb = c.jobs[(u >> 3) / c.nparts];
+            double sre, sim;
+            overlap_thread_sum<float>(c.f, nx, ny, jb, (u & 7) * 32 + lane, 256, part, c.nparts, sre, sim);
+            overlap_warp_reduce(sre, sim);
+            if (lane == 0) c.sums[u] = make_double2(sre, sim);
+        } else if (u < nov + c.src_units) {
+            mode_source_cells(c.src, (long long)(u - nov) * 32 + lane, (long long)c.src_units * 32,
+                              schedule_step(c.src, *c.step + c.s + 1));
+        } else {
+            int cell = (u - nov - c.src_units) * 32;
+            for (int b = 0; b < c.nstores; b++) {
+                const ChainStore &d = c.store[b];
+                if (cell >= 0 && cell < d.ncell) {
+                    const int t = d.t0 + d.dir * (int)(*c.step + c.s - 1), e = cell + lane;
+                    if (t >= 0 && t < d.duration && e < d.ncell) {
+                        const long long q = d.cells[e];
+                        float *dst = d.store + ((long long)t * d.ncell + e) * 3;
+#pragma unroll
+                        for (int m = 0; m < 3; m++) dst[m] = c.f[m][q];
+                    }
+                }
+                cell -= (d.ncell + 31) / 32 * 32;
+            }
+        }
+    }
+}
+
 template <bool CPML, bool LOSSY>
 __global__ void __launch_bounds__(kTileMaxThreads, 1)
-k_yee_tile(const __grid_constant__ StreamArgs a, const TileMaps *maps, const TileBox *tiles, TileShape sh, int *err)
+k_yee_tile(const __grid_constant__ StreamArgs a, const TileMaps *maps, const TileBox *tiles, TileShape sh,
+           const __grid_constant__ StepChain chain, int *err)
 {
     extern __shared__ __align__(128) float sm[];
     __shared__ TileSync sync;
     // programmatic dependent launch, as the other step kernels
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    auto after_previous = []() {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    };
+    if ((int)blockIdx.x == chain.ntiles) {
+        after_previous();
+        chain_add_up(chain.jobs, chain.njobs, chain.nparts, chain.prev, chain.scale, chain.dt, *chain.step + chain.s - 2,
+                     threadIdx.x >> 5, blockDim.x >> 5);
+        return;
+    }
     tile_sync_init(&sync);
-    yee_tile<CPML, LOSSY>(a, maps, tiles[blockIdx.x], sh, sm, &sync, err);
+    yee_tile<CPML, LOSSY>(a, maps, tiles[blockIdx.x], sh, sm, &sync, err, after_previous,
+                          [&]() { if ((int)blockIdx.x < chain.blocks) chain_units(chain, a.nx, a.ny); });
 }
 
-using TileKernel = void (*)(StreamArgs, const TileMaps *, const TileBox *, TileShape, int *);
+using TileKernel = void (*)(StreamArgs, const TileMaps *, const TileBox *, TileShape, StepChain, int *);
 
 static TileKernel tile_kernel(bool cpml, bool lossy)
 {
@@ -380,11 +426,13 @@ bool tile_make_maps(TileMaps *m, const float *const f[6], const float *cb, const
     return tma_encode_3d(&m->cb, cb, nx, ny, nz, bx, p.tp) && tma_encode_3d(&m->ca, ca ? ca : cb, nx, ny, nz, bx, p.tp);
 }
 
-void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *tiles, const TilePlan &p, int *err, cudaStream_t st)
+void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *tiles, const TilePlan &p, StepChain chain,
+                     int *err, cudaStream_t st)
 {
     note_launch(1);
+    chain.ntiles = (int)p.tiles.size();
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)p.tiles.size());
+    cfg.gridDim = dim3((unsigned)(chain.ntiles + (chain.prev ? 1 : 0)));
     cfg.blockDim = dim3((unsigned)p.threads);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
@@ -393,7 +441,7 @@ void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *t
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, tile_kernel(a.L > 0, a.ca[0] != nullptr), a, maps, tiles, TileShape{p.tp, p.sw}, err);
+    cudaLaunchKernelEx(&cfg, tile_kernel(a.L > 0, a.ca[0] != nullptr), a, maps, tiles, TileShape{p.tp, p.sw}, chain, err);
 }
 
 }  // namespace fdtd
