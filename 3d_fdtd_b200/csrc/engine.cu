@@ -1009,10 +1009,15 @@ static FlatArgs flat_args(Grid *g, double dt)
 
 static bool step_flat(Grid *g, double dt)
 {
-    const FlatArgs a = flat_args(g, dt);
+    FlatArgs a = flat_args(g, dt);
     const bool four = g->yee_variant != FDTD_YEE_FLAT && flat4_supported(g->nx, g->nz);
-    if (four) launch_flat4_step(a, g->st, g->side, g->ev_fork, g->ev_join);
-    else launch_flat_step(a, g->st, nullptr);
+    if (four) {
+        launch_flat4_step(a, g->st, g->side, g->ev_fork, g->ev_join);
+    } else {
+        if (g->mat_iso)   // equal arrays: read one
+            for (int c = 1; c < 3; c++) { a.cb[c] = a.cb[0]; a.ca[c] = a.ca[0]; }
+        launch_flat_step(a, g->st);
+    }
     CKL("flat step");
     return true;
 }

@@ -205,7 +205,7 @@ struct FlatArgs {
     int ring_k;
     long long ring_stride;
 };
-void launch_flat_step(const FlatArgs &a, cudaStream_t st, cudaEvent_t mid);
+void launch_flat_step(const FlatArgs &a, cudaStream_t st);
 int flat4_supported(int nx, int nz);
 // cells of one flat4 launch: planes kA..kA+nA-1 then kB.., `count` (group, row)
 // slots per plane laid out by region kind: 0 whole planes, 1 interior box
