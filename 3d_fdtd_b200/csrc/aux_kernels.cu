@@ -9,14 +9,44 @@
 namespace fdtd {
 
 // fixed amplitude and phase, or (sched != null) the schedule entry of step *step + offset
+// The small launches of a stepwise program stand between the step's kernels, each a
+// few us: all of them are programmatic dependents (launch_after), so that a launch is
+// set up while the one before it runs.  A step of a 64^3 grid that sets a source value
+// by a call: 21.5 us, 18 so.
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+static void launch_after(void (*k)(P...), dim3 grid, unsigned threads, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 __global__ void k_mode_source(SourceJob sj, double amplitude, double cph, double sph, const long long *step,
                               int step_offset)
 {
+    after_previous();
     const SrcStep v = sj.sched ? schedule_step(sj, *step + step_offset) : fixed_step(amplitude, cph, sph);
     mode_source_cells(sj, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, v);
 }
 
-__global__ void k_set_value(float *p, long long idx, float v) { p[idx] = v; }
+__global__ void k_set_value(float *p, long long idx, float v)
+{
+    after_previous();
+    p[idx] = v;
+}
 
 template <typename T>
 __global__ void k_overlap_partial(const T *const *Ex_, int nx, int ny, const OverlapJob *jobs, double2 *partials,
@@ -66,6 +96,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_overlap_now(const T *const *f, int nx, int ny, OverlapJob jb, double2 *partials,
                                                      unsigned *done, double scale, double2 *out)
 {
+    after_previous();
     overlap_block<T>(f, nx, ny, jb, blockIdx.x, gridDim.x, partials + blockIdx.x);
     __shared__ bool last;
     __shared__ double2 stage[64];
@@ -181,6 +212,7 @@ template <typename T>
 __global__ void k_dft(const T *const *f, int nx, int ny, int nz, int slice, int k_lo, int k_hi, double tr,
                       double ti, double2 *acc)
 {
+    after_previous();
     const long long nxy = (long long)nx * ny;
     long long cnt = slice >= 0 ? (long long)nx * (k_hi - k_lo) : nxy * (k_hi - k_lo);
     const long long accn = slice >= 0 ? (long long)nx * nz : nxy * nz;
@@ -229,6 +261,7 @@ template <typename T>
 __global__ void k_taper_store(const T *const *f, const long long *cells, int ncell, T *store, int t_index,
                               const long long *step, int t0, int dir, int duration)
 {
+    after_previous();
     int t = t_index;
     if (step) t = t0 + dir * (int)(*step);
     if (t < 0 || t >= duration) return;
@@ -331,7 +364,7 @@ void launch_mode_source_job(const SourceJob &sj_in, double amplitude, double cph
     SourceJob sj = sj_in;
     sj.win = mode_window(sj.nx, sj.ny, sj.cx, sj.cy, sj.mi, sj.mj, sj.ratio);
     note_launch();
-    k_mode_source<<<source_blocks(sj.win), 256, 0, st>>>(sj, amplitude, cph, sph, step, step_offset);
+    launch_after(k_mode_source, dim3((unsigned)source_blocks(sj.win)), 256, st, sj, amplitude, cph, sph, step, step_offset);
 }
 
 template <typename T>
@@ -368,7 +401,7 @@ template void launch_step_tail<double>(TailArgs, cudaStream_t);
 void launch_set_value(float *p, long long idx, float v, cudaStream_t st)
 {
     note_launch();
-    k_set_value<<<1, 1, 0, st>>>(p, idx, v);
+    launch_after(k_set_value, dim3(1), 1, st, p, idx, v);
 }
 
 // partials per overlap job: one 256-thread block per 256 window cells, 1 to 64
@@ -384,7 +417,7 @@ void launch_overlap_now(const T *const *f_dev, int nx, int ny, const OverlapJob 
 {
     note_launch();
     const int parts = overlap_parts((long long)job.win.wni * job.win.wnj);   // at most 64
-    k_overlap_now<T><<<parts, 256, 0, st>>>(f_dev, nx, ny, job, partials, done, scale, out);
+    launch_after(k_overlap_now<T>, dim3((unsigned)parts), 256, st, f_dev, nx, ny, job, partials, done, scale, out);
 }
 
 template <typename T>
@@ -409,7 +442,7 @@ void launch_dft(const T *const *f_dev, int nx, int ny, int nz, int slice, int k_
     int blocks = (int)((cnt + 255) / 256);
     if (blocks > 4736) blocks = 4736;
     note_launch();
-    k_dft<T><<<blocks, 256, 0, st>>>(f_dev, nx, ny, nz, slice, k_lo, k_hi, tr, ti, acc);
+    launch_after(k_dft<T>, dim3((unsigned)blocks), 256, st, f_dev, nx, ny, nz, slice, k_lo, k_hi, tr, ti, acc);
 }
 
 template <typename T>
@@ -435,7 +468,8 @@ void launch_taper_store(const T *const *f_dev, const long long *cells, int ncell
     int blocks = (ncell + 255) / 256;
     if (blocks > 592) blocks = 592;
     note_launch();
-    k_taper_store<T><<<blocks, 256, 0, st>>>(f_dev, cells, ncell, store, t_index, step, t0, dir, duration);
+    launch_after(k_taper_store<T>, dim3((unsigned)blocks), 256, st, f_dev, cells, ncell, store, t_index, step, t0, dir,
+                 duration);
 }
 
 template <typename T>

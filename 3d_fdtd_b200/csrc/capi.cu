@@ -44,7 +44,7 @@ template <typename T> bool launch_explicit_or_zsection(Grid *g, double dt, int e
     SourcePlanes s = source_table(g);
     const bool cpml = !expl && g->boundary == FDTD_BOUNDARY_CPML;
     if (efield) launch_update_E<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_e, cpml, expl, false, g->st);
-    else launch_update_H<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_m, true, cpml, expl, false, (T)g->dx, g->st);
+    else launch_update_H<T>(v, c, s, (T)dt, (T)(1 / (g->dx)), k_lo, k_hi, expl || g->sig_m, true, cpml, expl, false, g->st);
     return cuda_ok(cudaGetLastError(), "interior update");
 }
 

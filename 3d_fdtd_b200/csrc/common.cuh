@@ -62,6 +62,7 @@ struct GridView {
     const float *ep[3];
     const float *mu[3];
     const float *sig[6];    // null when every value is zero
+    const T *mur;           // factors of the Mur faces (yee_split.cu, mur_factor)
 };
 
 // CPML state.  Slab of axis a holds cells with index in [0,L) or [N-L,N) on

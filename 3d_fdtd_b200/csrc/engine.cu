@@ -362,7 +362,7 @@ Grid::~Grid()
         for (int m = 0; m < 6; m++) dfree(sig[m]);
         for (auto &p : planes) dfree(p.p);
         for (auto p : plane_pool) dfree(p);
-        dfree(d_step); dfree(d_done); dfree(d_jobs); dfree(d_partials);
+        dfree(d_step); dfree(d_done); dfree(d_mur); dfree(d_jobs); dfree(d_partials);
         dfree(wave.d_items); dfree(wave.d_cnt); dfree(wave.d_part); dfree(wave.d_ring);
         for (int s = 0; s < 2; s++)
             for (int e = 0; e < 2; e++)
@@ -399,6 +399,7 @@ template <typename T> GridView<T> view(Grid *g, int set)
     v.nx = g->nx; v.ny = g->ny; v.nz = g->nz; v.n = g->n;
     for (int m = 0; m < 6; m++) { v.f[m] = (T *)g->f[set][m]; v.old[m] = (T *)g->old[m]; v.sig[m] = g->sig[m]; }
     for (int c = 0; c < 3; c++) { v.ep[c] = g->ep[c]; v.mu[c] = g->mu[c]; }
+    v.mur = (const T *)g->d_mur;
     return v;
 }
 template GridView<float> view<float>(Grid *, int);
@@ -504,7 +505,7 @@ bool grid_upload_materials(Grid *g)
     g->sig_m = ((g->h_flag[9] | g->h_flag[10] | g->h_flag[11]) & 1) != 0;
     g->mat_iso = ((g->h_flag[1] | g->h_flag[2] | g->h_flag[7] | g->h_flag[8]) & 4) == 0;
     g->mat_dirty = 0;
-    g->coef_valid = false;
+    g->coef_valid = g->mur_valid = false;
     g->version++;
     return true;
 }
@@ -612,7 +613,7 @@ bool grid_set_precision(Grid *g, int prec)
         g->fields_from_host = true;
     }
     g->prec = prec;
-    g->coef_valid = false;
+    g->coef_valid = g->mur_valid = false;
     g->version++;
     return true;
 }
@@ -842,6 +843,15 @@ bool grid_prepare_step(Grid *g, double dt)
             g->pp_synced = true;
         }
     }
+    if (g->boundary == FDTD_BOUNDARY_MUR && (!g->mur_valid || g->mur_dt != dt)) {
+        if (!dalloc(&g->d_mur, (size_t)mur_table_size(g->nx, g->ny, g->nz) * sizeof(double), g->st, false)) return false;
+        if (g->prec == FDTD_F64) launch_mur_table<double>(view<double>(g, g->cur), (double *)g->d_mur, dt, g->dx, g->st);
+        else launch_mur_table<float>(view<float>(g, g->cur), (float *)g->d_mur, (float)dt, (float)g->dx, g->st);
+        CKL("Mur factors");
+        g->mur_valid = true;
+        g->mur_dt = dt;
+        g->version++;
+    }
     if (fast32_path(g)) {
         if (!g->coef_valid || g->coef_dt != dt) {
             size_t fb = (size_t)g->n * sizeof(float);
@@ -962,11 +972,11 @@ template <typename T> static bool step_split(Grid *g, double dt, bool extras)
     GridView<T> v = view<T>(g, g->cur);
     CpmlView<T> c = cpml_view<T>(g, g->cur);
     SourcePlanes s = source_table(g);
-    const T tdt = (T)dt, div = (T)(1 / (g->dx)), tdx = (T)g->dx;
+    const T tdt = (T)dt, div = (T)(1 / (g->dx));
     const bool cpml = g->boundary == FDTD_BOUNDARY_CPML;
     const bool mur = g->boundary == FDTD_BOUNDARY_MUR;
     launch_update_E<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_e, cpml, false, mur, g->st);
-    launch_update_H<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_m, g->mu_nonunit, cpml, false, mur, tdx, g->st);
+    launch_update_H<T>(v, c, s, tdt, div, 1, g->nz - 1, g->sig_m, g->mu_nonunit, cpml, false, mur, g->st);
     if (mur) {
         // a step by itself ends with this launch when nothing reads the counter after it
         StepEnd end{};
@@ -979,7 +989,7 @@ template <typename T> static bool step_split(Grid *g, double dt, bool extras)
             end.cap = g->probe_cap;
             end.count = g->d_probe_count;
         }
-        launch_mur_step<T>(v, tdt, tdx, end, g->st);
+        launch_mur_step<T>(v, end, g->st);
         CKL("step");
         g->step_ended = own;
         g->probes_done = end.np > 0;

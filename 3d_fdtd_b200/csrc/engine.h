@@ -122,6 +122,9 @@ struct Grid {
     float *cb[3] = {}, *ca[3] = {};
     double coef_dt = 0;
     bool coef_valid = false;
+    void *d_mur = nullptr;           // factors of the Mur faces (mur_factor), for mur_dt
+    double mur_dt = 0;
+    bool mur_valid = false;
     FusedMaps *fmaps[2] = {};        // TMA descriptors with set s as input (null: cp.async kernel)
     // one-pass streaming step (yee_stream.cu): tile plan of this grid's shape
     StreamPlan splan;

@@ -147,7 +147,7 @@ void launch_update_E(const GridView<T> &g, const CpmlView<T> &c, const SourcePla
                      int k_hi, bool sig, bool cpml, bool expl, bool snapshot, cudaStream_t st);
 template <typename T>
 void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor, int k_lo,
-                     int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, T dx, cudaStream_t st);
+                     int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, cudaStream_t st);
 template <typename T> void launch_save_shell(const GridView<T> &g, cudaStream_t st);
 template <typename T> void launch_mur(const GridView<T> &g, T dt, T dx, int efield, int ks, int ke, cudaStream_t st);
 // what the last launch of a step also does: record the probes, advance the counter (null: not)
@@ -161,7 +161,10 @@ struct StepEnd {
 };
 // The Mur faces of a whole step: launch_update_E with `snapshot`, launch_update_H
 // with `faces` (E's faces), launch_mur_step (H's)
-template <typename T> void launch_mur_step(const GridView<T> &g, T dt, T dx, const StepEnd &end, cudaStream_t st);
+template <typename T> void launch_mur_step(const GridView<T> &g, const StepEnd &end, cudaStream_t st);
+// the faces' factors, g.mur of the two
+long long mur_table_size(int nx, int ny, int nz);
+template <typename T> void launch_mur_table(const GridView<T> &g, T *out, T dt, T dx, cudaStream_t st);
 template <typename T> void launch_aos_to_soa(const double *aos, T *const d[6], long long n, cudaStream_t st);
 template <typename T> void launch_soa_to_aos(double *aos, T *const s[6], long long n, cudaStream_t st);
 

@@ -322,7 +322,7 @@ int timefield3d_set_spline_taper(timefield3d psi, double ep, double mu, int ncon
     cudaFree(d_edges);
     if (!ok) return fdtd_last_error();
     if (mu != 1.0) g->mu_nonunit = true;
-    g->coef_valid = false;
+    g->coef_valid = g->mur_valid = false;
     g->version++;
     return FDTD_OK;
 }

@@ -16,7 +16,7 @@
 // and a 64^3 grid had 128 blocks.  With a thread a cell the z and y neighbours
 // come from L2: FP64 steps of the 200 x 160 x 400 grid with a 12-cell CPML went
 // from 0.85 to 0.48 ms (the cells in no slab move 4.8 TB/s in E, 5.5 in H), and of
-// a 64^3 grid with the Mur boundary from 104 to 25 us.
+// a 64^3 grid with the Mur boundary from 104 to 25 us (18 now).
 // FP64 divisions cost as much as a third of the traffic: a cell whose three
 // permittivities are equal (every rasteriser writes them so) takes its
 // coefficient once.
@@ -75,7 +75,7 @@ __device__ __forceinline__ const float *src_of(const SourcePlanes &s, int k)
 // One block a plane walked its faces one after another, and the first and last
 // block a whole z face: 18.9 us for the E faces of a 64^3 grid and as much for
 // H's, and 24 us for the snapshot; as threads of the E and H updates, and in one
-// short launch after them, they are part of the 25 us of such a step.
+// short launch after them, they are part of the 18 us of such a step.
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T mur_scalar(const GridView<T> &g, int efield, int c, int axis, long long q, T dt, T dx)
@@ -86,6 +86,55 @@ __device__ __forceinline__ T mur_scalar(const GridView<T> &g, int efield, int c,
     const T mu = efield ? (T)g.mu[t][q] : (T)g.mu[c][q];
     const T sdt = A::mul(A::div((T)1, A::sqrt_(A::mul(ep, mu))), dt);
     return A::div(A::sub(sdt, dx), A::add(sdt, dx));
+}
+
+// The factors depend on the materials, dt and dx only, and a root and two divisions
+// each are most of a shell cell's latency, up to six in a row in FP64 (the H faces'
+// launch of a 64^3 grid 9.8 us, 5.9 with the factors read, its E faces in the H launch 13.9 and 9.2): a table, made when one
+// of the three changes.  Per axis and face: [E or H][low or high][tangential
+// component][cell of the face].
+__device__ __forceinline__ long long mur_face_cell(int axis, int nx, int ny, int i, int j, int k)
+{
+    return axis == 0 ? j + (long long)ny * k : i + (long long)nx * (axis == 1 ? k : j);
+}
+
+__host__ __device__ __forceinline__ long long mur_face(int axis, int nx, int ny, int nz)
+{
+    return axis == 0 ? (long long)ny * nz : (long long)nx * (axis == 1 ? nz : ny);
+}
+
+__device__ __forceinline__ long long mur_at(int nx, int ny, int nz, int efield, int c, int axis, int hi, int i, int j, int k)
+{
+    const long long before = axis == 0 ? 0 : mur_face(0, nx, ny, nz) + (axis == 1 ? 0 : mur_face(1, nx, ny, nz));
+    return 8 * before + (4 * (1 - efield) + 2 * hi + (c > axis ? c - 1 : c)) * mur_face(axis, nx, ny, nz) +
+           mur_face_cell(axis, nx, ny, i, j, k);
+}
+
+template <typename T>
+__device__ __forceinline__ T mur_factor(const GridView<T> &g, int efield, int c, int axis, int hi, int i, int j, int k)
+{
+    return g.mur[mur_at(g.nx, g.ny, g.nz, efield, c, axis, hi, i, j, k)];
+}
+
+template <typename T> __global__ void k_mur_table(GridView<T> g, T *out, T dt, T dx)
+{
+    const long long f0 = mur_face(0, g.nx, g.ny, g.nz), f1 = mur_face(1, g.nx, g.ny, g.nz), f2 = mur_face(2, g.nx, g.ny, g.nz);
+    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < 2 * (f0 + f1 + f2);
+         u += (long long)gridDim.x * blockDim.x) {
+        const int hi = (int)(u & 1);
+        long long t = u >> 1;
+        const int axis = t < f0 ? 0 : t < f0 + f1 ? 1 : 2;
+        if (axis >= 1) t -= f0;
+        if (axis == 2) t -= f1;
+        const int w = axis == 0 ? g.ny : g.nx, a = (int)(t % w), b = (int)(t / w);
+        const int i = axis == 0 ? hi * (g.nx - 1) : a;
+        const int j = axis == 0 ? a : axis == 1 ? hi * (g.ny - 1) : b;
+        const int k = axis == 2 ? hi * (g.nz - 1) : b;
+        const long long q = i + (long long)g.nx * (j + (long long)g.ny * k);
+        for (int c = 0; c < 3; c++)
+            for (int e = 0; e < 2 && c != axis; e++)
+                out[mur_at(g.nx, g.ny, g.nz, e, c, axis, hi, i, j, k)] = mur_scalar(g, e, c, axis, q, dt, dx);
+    }
 }
 
 template <typename T>
@@ -127,7 +176,7 @@ __host__ __device__ __forceinline__ long long mur_cells(int nx, int ny, int nz)
 
 // E (efield) or H of shell cell u
 template <typename T>
-__device__ __forceinline__ void mur_shell_cell(const GridView<T> &g, long long u, T dt, T dx, int efield)
+__device__ __forceinline__ void mur_shell_cell(const GridView<T> &g, long long u, int efield)
 {
     int i, j, k;
     shell_cell(u, g.nx, g.ny, g.nz, i, j, k);
@@ -141,17 +190,22 @@ __device__ __forceinline__ void mur_shell_cell(const GridView<T> &g, long long u
     auto component = [&](int c, int a, int fa, long long da, int b, int fb, long long db) {
         if (fa < 0 && fb < 0) return;
         const bool a_last = fa > fb;
+        const int last = a_last ? a : b, first = a_last ? b : a, f_last = a_last ? fa : fb, f_first = a_last ? fb : fa;
         const long long ql = q + (a_last ? da : db);
         const int m = efield ? c : 3 + c;
         const T *f = g.f[m], *old = g.old[m];
         T inner;
-        if ((a_last ? fb : fa) >= 0) {
+        if (f_first >= 0) {
             const long long qf = ql + (a_last ? db : da);
-            inner = mur_value(old[qf], mur_scalar(g, efield, c, a_last ? b : a, ql, dt, dx), f[qf], old[ql]);
+            const int in = f_last < 3 ? 1 : -1;   // ql: one step inwards along the last face's axis
+            inner = mur_value(old[qf],
+                              mur_factor(g, efield, c, first, f_first >= 3, i + (last == 0 ? in : 0),
+                                         j + (last == 1 ? in : 0), k + (last == 2 ? in : 0)),
+                              f[qf], old[ql]);
         } else {
             inner = f[ql];
         }
-        g.f[m][q] = mur_value(old[ql], mur_scalar(g, efield, c, a_last ? a : b, q, dt, dx), inner, old[q]);
+        g.f[m][q] = mur_value(old[ql], mur_factor(g, efield, c, last, f_last >= 3, i, j, k), inner, old[q]);
     };
     component(0, 1, fy, dy_, 2, fz, dz_);
     component(1, 0, fx, dx_, 2, fz, dz_);
@@ -414,14 +468,13 @@ k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, Cell
 // ---------------------------------------------------------------------------
 // h_coeff, h_main: 1/dt and 1/(1/dt), the coefficients where mu = 1 and no loss
 // MUR: the launch also sets E on the shell (the E faces of the Mur step): slots
-// past the planes are the shell's cells.  An interior cell whose +x, +y or +z
+// before the planes are the shell's cells.  An interior cell whose +x, +y or +z
 // neighbour is on the shell needs that face's new E and computes it itself --
 // such a neighbour lies on one face only, and its inner neighbour is the cell --
 // so H waits for no launch of its own between the two.
 template <typename T, bool SIG, bool MU, bool CPML, bool EXPL, int PART, bool MUR>
 __global__ void __launch_bounds__(kCellThreads, CPML ? 3 : 4)
-k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_coeff, T h_main, CellRange r, int slots,
-           T dx)
+k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_coeff, T h_main, CellRange r, int slots)
 {
     using A = Ar<T>;
     cell_prologue<PART>();
@@ -429,11 +482,11 @@ k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_
     const cell_t nxy = (cell_t)nx * (cell_t)ny;
     const int shell_slots = MUR ? (int)((mur_cells(nx, ny, nz) + gridDim.x * kCellThreads - 1) /
                                         (gridDim.x * kCellThreads)) : 0;
-    for (int slot = blockIdx.y; slot < slots + shell_slots; slot += gridDim.y) {
+    for (int slot = (int)blockIdx.y - shell_slots; slot < slots; slot += gridDim.y) {
         int i, j, k;
-        if (MUR && slot >= slots) {
-            const long long u = ((long long)(slot - slots) * gridDim.x + blockIdx.x) * kCellThreads + threadIdx.x;
-            if (u < mur_cells(nx, ny, nz)) mur_shell_cell(g, u, dt, dx, 1);
+        if (MUR && slot < 0) {   // the shell first: its cells take the longest
+            const long long u = ((long long)(slot + shell_slots) * gridDim.x + blockIdx.x) * kCellThreads + threadIdx.x;
+            if (u < mur_cells(nx, ny, nz)) mur_shell_cell(g, u, 1);
             continue;
         }
         if (!cell_of<PART>(r, nx, ny, nz, blockIdx.x * (unsigned)kCellThreads + threadIdx.x, slot, i, j, k)) continue;
@@ -442,7 +495,7 @@ k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_
         const T ex = g.f[0][q], ey = g.f[1][q], ez = g.f[2][q];
         T ex_j, ez_j, ex_k, ey_k, ey_i, ez_i;
         auto next = [&](int c, T inner, int axis, cell_t qn, bool face) -> T {
-            return MUR && face ? mur_value(g.old[c][q], mur_scalar(g, 1, c, axis, qn, dt, dx), inner, g.old[c][qn])
+            return MUR && face ? mur_value(g.old[c][q], mur_factor(g, 1, c, axis, 1, i, j, k), inner, g.old[c][qn])
                                : g.f[c][qn];
         };
         ex_j = next(0, ex, 1, q + nx, j == ny - 2);
@@ -612,7 +665,7 @@ __global__ void k_mur(GridView<T> g, T dt, T dx, int efield, int ks, int ke)
 // H faces of a step, the probes (interior ones: no face sets them) and the step
 // counter
 template <typename T>
-__global__ void __launch_bounds__(kCellThreads) k_mur_step(GridView<T> g, T dt, T dx, StepEnd end)
+__global__ void __launch_bounds__(kCellThreads) k_mur_step(GridView<T> g, StepEnd end)
 {
     cell_prologue<0>();
     if (blockIdx.x == gridDim.x - 1) {
@@ -625,7 +678,7 @@ __global__ void __launch_bounds__(kCellThreads) k_mur_step(GridView<T> g, T dt, 
         return;
     }
     const long long u = blockIdx.x * (long long)kCellThreads + threadIdx.x;
-    if (u < mur_cells(g.nx, g.ny, g.nz)) mur_shell_cell(g, u, dt, dx, 0);
+    if (u < mur_cells(g.nx, g.ny, g.nz)) mur_shell_cell(g, u, 0);
 }
 
 // AoS double (reference layout) -> SoA T, whole grid
@@ -720,7 +773,7 @@ void launch_update_E(const GridView<T> &g, const CpmlView<T> &c, const SourcePla
 
 template <typename T>
 void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePlanes &s, T dt, T divisor,
-                     int k_lo, int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, T dx, cudaStream_t st)
+                     int k_lo, int k_hi, bool sig, bool mu, bool cpml, bool expl, bool faces, cudaStream_t st)
 {
     const CellRange all = cell_range(g.nx, g.ny, g.nz, k_lo, k_hi, false);
     const T h_coeff = (T)1 / dt, h_main = (T)1 / h_coeff;
@@ -728,7 +781,7 @@ void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePla
 #define FDTD_H(RANGE, ...)                                                                                          \
     for_range(RANGE, g.nx, g.ny, g.nz, part, [&](dim3 grd, int slots) {                                             \
         if (faces) grd.y = (unsigned)std::min<long long>(65535, grd.y + mur_cells(g.nx, g.ny, g.nz) / ((long long)grd.x * kCellThreads) + 1); \
-        launch_cells(k_update_H<T, __VA_ARGS__>, grd, st, g, c, s, dt, divisor, h_coeff, h_main, RANGE, slots, dx); \
+        launch_cells(k_update_H<T, __VA_ARGS__>, grd, st, g, c, s, dt, divisor, h_coeff, h_main, RANGE, slots); \
     })
 #define FDTD_H3(RANGE, CP, PT, FACES)                                     \
     do {                                                                  \
@@ -752,10 +805,22 @@ void launch_update_H(const GridView<T> &g, const CpmlView<T> &c, const SourcePla
 #undef FDTD_H
 }
 
-template <typename T> void launch_mur_step(const GridView<T> &g, T dt, T dx, const StepEnd &end, cudaStream_t st)
+template <typename T> void launch_mur_step(const GridView<T> &g, const StepEnd &end, cudaStream_t st)
 {
     const long long blocks = (mur_cells(g.nx, g.ny, g.nz) + kCellThreads - 1) / kCellThreads + 1;
-    launch_cells(k_mur_step<T>, dim3((unsigned)blocks), st, g, dt, dx, end);
+    launch_cells(k_mur_step<T>, dim3((unsigned)blocks), st, g, end);
+}
+
+long long mur_table_size(int nx, int ny, int nz)
+{
+    return 8 * (mur_face(0, nx, ny, nz) + mur_face(1, nx, ny, nz) + mur_face(2, nx, ny, nz));
+}
+
+template <typename T> void launch_mur_table(const GridView<T> &g, T *out, T dt, T dx, cudaStream_t st)
+{
+    note_launch();
+    const long long blocks = (mur_table_size(g.nx, g.ny, g.nz) / 4 + 255) / 256;
+    k_mur_table<T><<<(unsigned)std::min<long long>(blocks, 4736), 256, 0, st>>>(g, out, dt, dx);
 }
 
 template <typename T>
@@ -796,9 +861,10 @@ void launch_soa_to_aos(double *aos, T *const s[6], long long n, cudaStream_t st)
 #define FDTD_INST(T)                                                                                          \
     template void launch_update_E<T>(const GridView<T> &, const CpmlView<T> &, const SourcePlanes &, T, T, int, \
                                      int, bool, bool, bool, bool, cudaStream_t);                               \
-    template void launch_mur_step<T>(const GridView<T> &, T, T, const StepEnd &, cudaStream_t);                \
+    template void launch_mur_step<T>(const GridView<T> &, const StepEnd &, cudaStream_t);                     \
+    template void launch_mur_table<T>(const GridView<T> &, T *, T, T, cudaStream_t);                          \
     template void launch_update_H<T>(const GridView<T> &, const CpmlView<T> &, const SourcePlanes &, T, T, int, \
-                                     int, bool, bool, bool, bool, bool, T, cudaStream_t);                      \
+                                     int, bool, bool, bool, bool, bool, cudaStream_t);                         \
     template void launch_save_shell<T>(const GridView<T> &, cudaStream_t);                                    \
     template void launch_mur<T>(const GridView<T> &, T, T, int, int, int, cudaStream_t);                       \
     template void launch_aos_to_soa<T>(const double *, T *const[6], long long, cudaStream_t);                  \
