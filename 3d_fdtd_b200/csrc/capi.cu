@@ -5,6 +5,8 @@
 // on the GPU.  Every entry point takes the API lock, records failures with
 // set_error (never aborts) and returns.
 #include <algorithm>
+#include <atomic>
+#include <thread>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -303,6 +305,40 @@ timefield3d timefield3d_copy(timefield3d psi)
     return c;
 }
 
+// The mirrors of a grid are 192 B a cell, and one thread clears 14 GB/s: 6.8 ms for
+// 96x80x64 cells, more than the 256 steps between two calls take; up to eight share
+// it, 1.9 ms.  Threads that cannot be started are done without.
+namespace {
+struct HostSpan {
+    char *p;
+    size_t bytes;
+};
+void zero_host(const HostSpan *span, int n)
+{
+    constexpr size_t kPiece = 1 << 20;
+    constexpr int kThreads = 8;
+    size_t total = 0;
+    for (int i = 0; i < n; i++) total += (span[i].bytes + kPiece - 1) / kPiece;
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+        for (size_t u; (u = next.fetch_add(1)) < total;) {
+            int i = 0;
+            for (size_t m; u >= (m = (span[i].bytes + kPiece - 1) / kPiece); i++) u -= m;
+            memset(span[i].p + u * kPiece, 0, std::min(kPiece, span[i].bytes - u * kPiece));
+        }
+    };
+    std::thread t[kThreads - 1];
+    int started = 0;
+    const int want = (int)std::min<size_t>(kThreads - 1, total / 8);   // 8 MB or more for a thread
+    try {
+        for (; started < want; started++) t[started] = std::thread(work);
+    } catch (const std::exception &) {
+    }
+    work();
+    for (int i = 0; i < started; i++) t[i].join();
+}
+}  // namespace
+
 void timefield3d_zero_fields(timefield3d psi)
 {
     LOCK;
@@ -314,11 +350,15 @@ void timefield3d_zero_fields(timefield3d psi)
     // sync may have written
     size_t n = (size_t)psi.i * psi.j * psi.k;
     if (!g->dev || g->host_mirror_written) {
-        memset(psi.fields, 0, 6 * n * sizeof(double));
-        memset(psi.old_fields, 0, 6 * n * sizeof(double));
-        memset(psi.fourier_fields, 0, 6 * n * sizeof(complex));
+        const HostSpan mirrors[] = {{(char *)psi.fields, 6 * n * sizeof(double)},
+                                    {(char *)psi.old_fields, 6 * n * sizeof(double)},
+                                    {(char *)psi.fourier_fields, 6 * n * sizeof(complex)}};
+        zero_host(mirrors, 3);
     }
-    if (!g->dev || g->host_sources_written) memset(psi.sources, 0, 6 * n * sizeof(float));
+    if (!g->dev || g->host_sources_written) {
+        const HostSpan sources{(char *)psi.sources, 6 * n * sizeof(float)};
+        zero_host(&sources, 1);
+    }
     g->host_mirror_written = false;
     g->host_sources_written = false;
     g->fields_from_host = false;
