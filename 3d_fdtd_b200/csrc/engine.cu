@@ -400,6 +400,8 @@ template <typename T> GridView<T> view(Grid *g, int set)
     for (int m = 0; m < 6; m++) { v.f[m] = (T *)g->f[set][m]; v.old[m] = (T *)g->old[m]; v.sig[m] = g->sig[m]; }
     for (int c = 0; c < 3; c++) { v.ep[c] = g->ep[c]; v.mu[c] = g->mu[c]; }
     v.mur = (const T *)g->d_mur;
+    if (g->mat_iso)   // equal arrays: read one
+        for (int c = 1; c < 3; c++) v.ep[c] = v.ep[0];
     return v;
 }
 template GridView<float> view<float>(Grid *, int);
