@@ -470,7 +470,8 @@ static bool upload_deinterleave(Grid *g, const float *host, int stride, float **
 bool grid_upload_materials(Grid *g)
 {
     // only the arrays the rasterisers touched (kMatEp / kMatMu / kMatSig bits);
-    // flags: [0..2] ep != 1, [3..5] mu != 1, [6..11] sig != 0 (bit 2: not finite)
+    // flags: [0..2] ep != 1, [3..5] mu != 1, [6..11] sig != 0 (bit 2: not finite; bit 4: see
+    // k_deinterleave)
     const int dirty = g->mat_dirty;
     // Pin the host material mirrors once a grid uploads them a second time
     // (design loops re-rasterise and re-upload every evaluation); a grid
