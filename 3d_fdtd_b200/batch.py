@@ -253,7 +253,8 @@ def _sweep_call(fd, slots, nsteps, steps_per_launch, band_rows, tiles_per_sm):
 
 def autotune_tiles(fd, cands: list[dict], steps: int = 128, steps_per_launch: int = 64,
                    shapes=((0, 2.0), (0, 4.0), (0, 8.0), (4, 4.0), (3, 4.0))) -> tuple[tuple[int, float], dict]:
-    """Tile shape of the persistent sweep: for each (band rows cap, tiles per
+    """Tile shape of the persistent launches (grids whose coefficients differ take
+    them; others are not shaped by it): for each (band rows cap, tiles per
     SM) the sweep of these candidates runs `steps` steps after a warm-up, timed
     on the host around a synchronised call; the fastest shape is returned."""
     slots = []
@@ -281,9 +282,8 @@ def autotune_tiles(fd, cands: list[dict], steps: int = 128, steps_per_launch: in
 
 def sweep_persistent(fd, cands: list[dict], group: int = 8, steps_per_launch: int = 64,
                      shape: tuple[int, float] | None = None) -> dict:
-    """Every candidate through persistent sweep launches: candidates sorted by
-    step count, `group` at a time advance together (uneven lengths inside the
-    launches); the next group is set up on the host while the current one runs."""
+    """Every candidate through fdtd_sweep_run: candidates sorted by step count,
+    `group` at a time advance together (of uneven lengths); the next group is set up on the host while the current one runs."""
     if not cands:
         return dict(results={}, amplitudes={}, seconds=0.0, cell_steps=0, bytes=0, shape=None, tuning={})
     order = sorted(cands, key=lambda c: c["steps"])
@@ -332,7 +332,7 @@ def main():
     ap.add_argument("--seed", type=int, default=2)
     ap.add_argument("--steps-scale", type=float, default=1.0)
     ap.add_argument("--mode", choices=["persistent", "slots"], default="persistent",
-                    help="persistent: groups of candidates in persistent sweep launches; slots: one run per slot")
+                    help="persistent: groups of candidates in one sweep call each; slots: one run per slot")
     ap.add_argument("--group", type=int, default=8)
     args = ap.parse_args()
     import torch
