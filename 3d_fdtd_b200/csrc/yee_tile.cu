@@ -19,9 +19,9 @@
 //  - all columns are cut at the same planes, in one or two waves of blocks: tiles
 //    that run side by side read a shared halo row from DRAM once (kInStep below).
 // Per step, before (three coefficients, cp.async) and now: 200x160x400 with CPML 189
-// and 160 us (5.0 TB/s of the 52 B a cell alone), with PEC 144 and 120 us; 384x256x384
-// CPML 792 and 415; 256x128x128 CPML 77 and 67; 96x80x64 CPML, conductivity 45 and
-// 14.5 us.  Two blocks an SM (96 registers) spill with CPML and gave nothing without.
+// and 158 us (5.05 TB/s of algorithmic bytes), with PEC 144 and 115 us; 384x256x384
+// CPML 792 and 414; 256x128x128 CPML 77 and 67; 96x80x64 CPML, conductivity 45 and
+// 14 us.  Two blocks an SM (96 registers) spill with CPML and gave nothing without.
 #include "tile_cells.cuh"
 #include "plane_ops.cuh"
 
@@ -86,6 +86,9 @@ k_yee_tile(const __grid_constant__ StreamArgs a, const TileMaps *maps, const Til
         return;
     }
     tile_sync_init(&sync);
+    // the descriptors, while the previous launch ends (0.3 us of a step)
+    if (threadIdx.x < sizeof(TileMaps) / sizeof(CUtensorMap))
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<const CUtensorMap *>(maps) + threadIdx.x) : "memory");
     yee_tile<CPML, LOSSY>(a, maps, tiles[blockIdx.x], sh, sm, &sync, err, after_previous,
                           [&]() { if ((int)blockIdx.x < chain.blocks) chain_units(chain, a.nx, a.ny); });
 }
