@@ -1,5 +1,6 @@
 // yee_stream.cu -- FP32 Yee step in one pass: E^{n+1} and H^{n+3/2} of every
-// cell in a single launch, streaming z-planes through shared memory.
+// cell in a single launch, streaming z-planes through shared memory, for grids whose
+// three E coefficients differ in some cell (yee_tile.cu takes the others).
 //
 // Why one pass.  Updating E and H in two launches reads each field set twice
 // per step (the E launch reads H, the H launch reads the new E), about 84 B per

@@ -1,5 +1,6 @@
 // yee_sweep.cu -- many grids (taper candidates of uneven length) advanced
-// together by one persistent launch per chunk of steps.
+// together by one persistent launch per chunk of steps, for grids whose three E
+// coefficients differ in some cell (the others run on their own streams, run_sweep).
 //
 // The reference simulates one design at a time (3d_fdtd.c:93-202).  An
 // optimisation sweep runs many independent candidates; here every resident

@@ -230,8 +230,9 @@ enum fdtd_precision { FDTD_F64 = 0, FDTD_F32 = 1 };
  * L2; runs with probes or bound taper stores, and single steps, use flat4).
  * stream (one launch per step: each thread block streams a band of rows
  * through its planes, E and H of a plane in one pass, reading each array once
- * and writing the other field set; nx % 4 == 0, fewer than 2^31 cells).  AUTO picks stream where the
- * grid allows it, else flat4 where nx allows, else flat.  wave's fields are
+ * and writing the other field set; nx % 4 == 0, fewer than 2^31 cells; one
+ * kernel for grids whose E coefficients agree on a cell's components, one for the
+ * others).  AUTO picks stream where the grid allows it, else flat4 where nx allows, else flat.  wave's fields are
  * bit-identical to flat4's; stream's agree with flat4's to float rounding. */
 enum fdtd_yee_variant {
     FDTD_YEE_AUTO = 0, FDTD_YEE_FLAT = 1, FDTD_YEE_FUSED = 2, FDTD_YEE_FLAT4 = 3, FDTD_YEE_WAVE = 4,
@@ -271,8 +272,8 @@ int timefield3d_set_wave_steps(timefield3d psi, int steps_per_launch, int steps_
  * and the ticket total, or -1 on invalid input. */
 int fdtd_wave_schedule(int nx, int ny, int nz, int cpml_cells, int steps, int sweep, int blocks_per_ticket,
                        const int *job_z, int njobs, int nparts, int *out, int cap, int *tickets);
-/* The tile plan of the FDTD_YEE_STREAM kernel (host computation, no device
- * work), for inspection and tests.  No reference counterpart.  Grid
+/* The tile plan of the FDTD_YEE_STREAM kernel for grids whose coefficients
+ * differ on a cell's components (host computation, no device work), for inspection and tests.  No reference counterpart.  Grid
  * nx x ny x nz, CPML thickness (0: none), lossy != 0 when the E update has
  * loss coefficients, nsm streaming multiprocessors.  Writes 4 ints per tile
  * into tiles (capacity cap tiles; null to count): first owned row, owned rows,
