@@ -34,19 +34,13 @@ constexpr int kCellThreads = 256;
 using cell_t = unsigned;
 
 // Programmatic dependent launch: wait for the previous kernel's results, and let
-// the next one's blocks be set up meanwhile (they wait in turn).  PART 2 of an
-// update does not depend on PART 1, only on what PART 1 waited for before it let
-// this launch start: it works at once and waits for PART 1 at its end, so that
-// whoever waits for it waits for both.
-template <int PART> __device__ __forceinline__ void cell_prologue()
+// the next one's blocks be set up meanwhile (they wait in turn).  Every kernel does
+// both before it touches the fields: only its own wait makes earlier launches'
+// writes visible to it.  (The two launches of a CPML update do not depend on each
+// other, but on what came before both; the second used to wait at its end only,
+// which saved 3.6 us of a 200 x 160 x 400 step's 476.6 and rested on no promise.)
+__device__ __forceinline__ void after_previous()
 {
-    if (PART == 2) return;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-template <int PART> __device__ __forceinline__ void cell_epilogue()
-{
-    if (PART != 2) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -401,7 +395,7 @@ __global__ void __launch_bounds__(kCellThreads, CPML ? 3 : 4)
 k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, CellRange r, int slots)
 {
     using A = Ar<T>;
-    cell_prologue<PART>();
+    after_previous();
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const cell_t nxy = (cell_t)nx * (cell_t)ny;
     for (int slot = blockIdx.y; slot < slots; slot += gridDim.y) {
@@ -458,7 +452,6 @@ k_update_E(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, Cell
         for (int m = 0; m < 3; m++) g.f[m][q] = e[m];
         if (CPML) cpml_store(p, c, 0);
     }
-    cell_epilogue<PART>();
 }
 
 // ---------------------------------------------------------------------------
@@ -478,7 +471,7 @@ __global__ void __launch_bounds__(kCellThreads, CPML ? 3 : 4)
 k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_coeff, T h_main, CellRange r, int slots)
 {
     using A = Ar<T>;
-    cell_prologue<PART>();
+    after_previous();
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const cell_t nxy = (cell_t)nx * (cell_t)ny;
     const int shell_slots = MUR ? (int)((mur_cells(nx, ny, nz) + gridDim.x * kCellThreads - 1) /
@@ -543,7 +536,6 @@ k_update_H(GridView<T> g, CpmlView<T> c, SourcePlanes src, T dt, T divisor, T h_
         for (int m = 0; m < 3; m++) g.f[3 + m][q] = h[m];
         if (CPML) cpml_store(p, c, 1);
     }
-    cell_epilogue<PART>();
 }
 
 // ---------------------------------------------------------------------------
@@ -670,7 +662,7 @@ __global__ void k_mur(GridView<T> g, T dt, T dx, int efield, int ks, int ke)
 template <typename T>
 __global__ void __launch_bounds__(kCellThreads) k_mur_step(GridView<T> g, StepEnd end)
 {
-    cell_prologue<0>();
+    after_previous();
     if (blockIdx.x == gridDim.x - 1) {
         for (int p = threadIdx.x; p < end.np; p += kCellThreads) {
             const int n = end.count[p];
@@ -710,7 +702,7 @@ __global__ void k_soa_to_aos(double *aos, const T *s0, const T *s1, const T *s2,
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-// launch with a programmatic dependency on the preceding kernel (cell_prologue)
+// launch with a programmatic dependency on the preceding kernel (after_previous)
 template <typename... P, typename... A>
 static void launch_cells(void (*k)(P...), dim3 grid, cudaStream_t st, A... args)
 {
