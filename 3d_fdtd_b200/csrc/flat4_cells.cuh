@@ -3,12 +3,11 @@
 // the per-field launches (yee_flat4.cu) and the multi-step wavefront kernel
 // (yee_wave.cu).
 //
-// COH selects how the field arrays are read.  Within one per-field launch no
-// block writes what another block reads, so the fields go through the
-// read-only (non-coherent) path.  In the wavefront kernel other blocks of the
-// same launch write the fields a block reads (after an acquire on their
-// completion count), so every field load is a plain coherent load there; the
-// coefficients, profiles and source planes stay read-only either way.
+// Fields, auxiliaries and source planes go through plain loads: another launch
+// writes them while this one's blocks may already be resident (programmatic
+// dependent launch), and in the wavefront kernel other blocks of the same launch do.
+// The read-only path (ldv, __ldg) is for what no kernel of a run writes:
+// coefficients and profiles.
 #pragma once
 
 #include "common.cuh"
@@ -48,19 +47,6 @@ template <int W> __device__ __forceinline__ Vf<W> ldv_rw(const float *p)
         r.v[0] = *p;
     }
     return r;
-}
-
-// field loads: read-only path (COH false) or plain coherent loads (COH true)
-template <int W, bool COH> __device__ __forceinline__ Vf<W> ldf(const float *p)
-{
-    if constexpr (COH) return ldv_rw<W>(p);
-    else return ldv<W>(p);
-}
-
-template <bool COH> __device__ __forceinline__ float ldf1(const float *p)
-{
-    if constexpr (COH) return *p;
-    else return __ldg(p);
 }
 
 template <int W> __device__ __forceinline__ void stv(float *p, const Vf<W> &x)
@@ -259,7 +245,7 @@ __device__ __forceinline__ void locate(const Region4 &r, int ngroups, int ny, in
 
 // E update of the W cells of group g, row j, plane k (all lanes of the warp
 // call it); ls: step within a multi-step launch (selects the source ring entry)
-template <int W, int SLABS, bool LOSSY, bool COH = false>
+template <int W, int SLABS, bool LOSSY>
 __device__ __forceinline__ void e_cells(const FlatArgs &a, int g, int j, int k, bool live, int ls = 0)
 {
     constexpr bool CPML = SLABS != 0;
@@ -274,8 +260,8 @@ __device__ __forceinline__ void e_cells(const FlatArgs &a, int g, int j, int k, 
     // ---- phase 1: loads
     Vf<W> hy = fillv<W>(0.f), hz = hy;
     if (live) {
-        hy = ldf<W, COH>(a.f[4] + q0);
-        hz = ldf<W, COH>(a.f[5] + q0);
+        hy = ldv_rw<W>(a.f[4] + q0);
+        hz = ldv_rw<W>(a.f[5] + q0);
     }
     // the i-1 neighbour of element 0 is lane-1's last element when lane-1 holds group g-1
     float hy_im0 = __shfl_up_sync(0xffffffffu, hy.v[W - 1], 1);
@@ -283,12 +269,12 @@ __device__ __forceinline__ void e_cells(const FlatArgs &a, int g, int j, int k, 
     const int key_prev = __shfl_up_sync(0xffffffffu, key, 1);
     if (!live) return;
     if (lane == 0 || g == 0 || key_prev != key - 1) {
-        hy_im0 = g > 0 ? ldf1<COH>(a.f[4] + q0 - 1) : 0.f;
-        hz_im0 = g > 0 ? ldf1<COH>(a.f[5] + q0 - 1) : 0.f;
+        hy_im0 = g > 0 ? a.f[4][q0 - 1] : 0.f;
+        hz_im0 = g > 0 ? a.f[5][q0 - 1] : 0.f;
     }
-    const Vf<W> hx = ldf<W, COH>(a.f[3] + q0);
-    const Vf<W> hx_jm = ldf<W, COH>(a.f[3] + q0 - nx), hz_jm = ldf<W, COH>(a.f[5] + q0 - nx);
-    const Vf<W> hx_km = ldf<W, COH>(a.f[3] + q0 - nxy), hy_km = ldf<W, COH>(a.f[4] + q0 - nxy);
+    const Vf<W> hx = ldv_rw<W>(a.f[3] + q0);
+    const Vf<W> hx_jm = ldv_rw<W>(a.f[3] + q0 - nx), hz_jm = ldv_rw<W>(a.f[5] + q0 - nx);
+    const Vf<W> hx_km = ldv_rw<W>(a.f[3] + q0 - nxy), hy_km = ldv_rw<W>(a.f[4] + q0 - nxy);
     const Vf<W> b0 = ldv<W>(a.cb[0] + q0), b1 = ldv<W>(a.cb[1] + q0), b2 = ldv<W>(a.cb[2] + q0);
     Vf<W> ex = ldv_rw<W>(a.f[0] + q0), ey = ldv_rw<W>(a.f[1] + q0), ez = ldv_rw<W>(a.f[2] + q0);
     Vf<W> c0 = fillv<W>(1.f), c1 = c0, c2 = c0;
@@ -329,9 +315,9 @@ __device__ __forceinline__ void e_cells(const FlatArgs &a, int g, int j, int k, 
             cx = c.x; cy = c.y; cz = c.z;
         }
         if (sp) {
-            cx -= dx * __ldg(sp + ij0 + e);
-            cy -= dx * __ldg(sp + nxy + ij0 + e);
-            cz -= dx * __ldg(sp + 2 * nxy + ij0 + e);
+            cx -= dx * sp[ij0 + e];
+            cy -= dx * sp[nxy + ij0 + e];
+            cz -= dx * sp[2 * nxy + ij0 + e];
         }
         ex.v[e] = c0.v[e] * ex.v[e] + b0.v[e] * cx;
         ey.v[e] = c1.v[e] * ey.v[e] + b1.v[e] * cy;
@@ -348,7 +334,7 @@ __device__ __forceinline__ void e_cells(const FlatArgs &a, int g, int j, int k, 
 }
 
 // H update of the W cells of group g, row j, plane k (all lanes of the warp call it)
-template <int W, int SLABS, bool COH = false>
+template <int W, int SLABS>
 __device__ __forceinline__ void h_cells(const FlatArgs &a, int g, int j, int k, bool live, int ls = 0)
 {
     constexpr bool CPML = SLABS != 0;
@@ -362,8 +348,8 @@ __device__ __forceinline__ void h_cells(const FlatArgs &a, int g, int j, int k, 
     // ---- phase 1: loads
     Vf<W> ey = fillv<W>(0.f), ez = ey;
     if (live) {
-        ey = ldf<W, COH>(a.f[1] + q0);
-        ez = ldf<W, COH>(a.f[2] + q0);
+        ey = ldv_rw<W>(a.f[1] + q0);
+        ez = ldv_rw<W>(a.f[2] + q0);
     }
     // the i+1 neighbour of the last element is lane+1's element 0 when lane+1 holds group g+1
     float ey_ipw = __shfl_down_sync(0xffffffffu, ey.v[0], 1);
@@ -371,12 +357,12 @@ __device__ __forceinline__ void h_cells(const FlatArgs &a, int g, int j, int k, 
     const int key_next = __shfl_down_sync(0xffffffffu, key, 1);
     if (!live) return;
     if (lane == 31 || g == ngroups - 1 || key_next != key + 1) {
-        ey_ipw = g < ngroups - 1 ? ldf1<COH>(a.f[1] + q0 + W) : 0.f;
-        ez_ipw = g < ngroups - 1 ? ldf1<COH>(a.f[2] + q0 + W) : 0.f;
+        ey_ipw = g < ngroups - 1 ? a.f[1][q0 + W] : 0.f;
+        ez_ipw = g < ngroups - 1 ? a.f[2][q0 + W] : 0.f;
     }
-    const Vf<W> ex = ldf<W, COH>(a.f[0] + q0);
-    const Vf<W> ex_jp = ldf<W, COH>(a.f[0] + q0 + nx), ez_jp = ldf<W, COH>(a.f[2] + q0 + nx);
-    const Vf<W> ex_kp = ldf<W, COH>(a.f[0] + q0 + nxy), ey_kp = ldf<W, COH>(a.f[1] + q0 + nxy);
+    const Vf<W> ex = ldv_rw<W>(a.f[0] + q0);
+    const Vf<W> ex_jp = ldv_rw<W>(a.f[0] + q0 + nx), ez_jp = ldv_rw<W>(a.f[2] + q0 + nx);
+    const Vf<W> ex_kp = ldv_rw<W>(a.f[0] + q0 + nxy), ey_kp = ldv_rw<W>(a.f[1] + q0 + nxy);
     Vf<W> hx = ldv_rw<W>(a.f[3] + q0), hy = ldv_rw<W>(a.f[4] + q0), hz = ldv_rw<W>(a.f[5] + q0);
     const float *sp = step_src_plane(a, k, ls);
     XSlab<W> xs;
@@ -409,9 +395,9 @@ __device__ __forceinline__ void h_cells(const FlatArgs &a, int g, int j, int k, 
             cx = c.x; cy = c.y; cz = c.z;
         }
         if (sp) {
-            cx += dx * __ldg(sp + 3 * nxy + ij0 + e);
-            cy += dx * __ldg(sp + 4 * nxy + ij0 + e);
-            cz += dx * __ldg(sp + 5 * nxy + ij0 + e);
+            cx += dx * sp[3 * nxy + ij0 + e];
+            cy += dx * sp[4 * nxy + ij0 + e];
+            cz += dx * sp[5 * nxy + ij0 + e];
         }
         hx.v[e] = hx.v[e] - hb * cx;
         hy.v[e] = hy.v[e] - hb * cy;

@@ -112,11 +112,9 @@ __device__ __forceinline__ void stream_profile_table(float *pt, const StreamArgs
     }
 }
 
-// COH: plain (coherent) loads, for launches in which other blocks wrote the
-// auxiliaries (the multi-step sweep); else the read-only path
 // (a single x-slab cell, W = 1, also takes its y and z profiles from the
 // tile's table `pt` here, an iteration before they are used)
-template <int W, int A0, bool COH>
+template <int W, int A0>
 __device__ __forceinline__ void stream_yzpsi_load(YZPsi<W> &s, const StreamArgs &a, int i0, int j, int k,
                                                   sidx_t ij0, sidx_t nxy, const float *pt = nullptr)
 {
@@ -126,8 +124,8 @@ __device__ __forceinline__ void stream_yzpsi_load(YZPsi<W> &s, const StreamArgs 
     s.pxy = fillv<W>(0.f); s.pzy = s.pxy; s.pxz = s.pxy; s.pyz = s.pxy;
     if (s.sj >= 0) {
         const sidx_t sy = (sidx_t)i0 + (sidx_t)nx * (sidx_t)(s.sj + 2 * L * k);
-        s.pxy = ldf<W, COH>(a.psi_in[1][A0] + sy);
-        s.pzy = ldf<W, COH>(a.psi_in[1][A0 + 1] + sy);
+        s.pxy = ldv_rw<W>(a.psi_in[1][A0] + sy);
+        s.pzy = ldv_rw<W>(a.psi_in[1][A0 + 1] + sy);
         if constexpr (W == 1) {
             const float *py = pt + (6 + 3 * (A0 / 2)) * 2 * L + s.sj;
 #pragma unroll
@@ -136,8 +134,8 @@ __device__ __forceinline__ void stream_yzpsi_load(YZPsi<W> &s, const StreamArgs 
     }
     if (s.sk >= 0) {
         const sidx_t sz = ij0 + nxy * (sidx_t)s.sk;
-        s.pxz = ldf<W, COH>(a.psi_in[2][A0] + sz);
-        s.pyz = ldf<W, COH>(a.psi_in[2][A0 + 1] + sz);
+        s.pxz = ldv_rw<W>(a.psi_in[2][A0] + sz);
+        s.pyz = ldv_rw<W>(a.psi_in[2][A0 + 1] + sz);
         if constexpr (W == 1) {
             const float *pz = pt + (12 + 3 * (A0 / 2)) * 2 * L + s.sk;
 #pragma unroll
@@ -291,7 +289,7 @@ __host__ __device__ inline StreamRoles stream_roles(int nx, int L, int tp)
 // x-slab cell, W = 1).  X: x-slab group (x terms, and the cells x = 0 / nx-1
 // of the row ends stay); EDGE: the group may hold x = 0 / nx-1 (row ends of a
 // grid without CPML).  hy_im0, hz_im0: Hy, Hz at x = i0 - 1.
-template <int W, bool X, bool EDGE, bool CPML, bool LOSSY, bool COH>
+template <int W, bool X, bool EDGE, bool CPML, bool LOSSY>
 __device__ __forceinline__ void stream_e_group(Vf<W> &ex, Vf<W> &ey, Vf<W> &ez, const Vf<W> &hx, const Vf<W> &hy,
                                                const Vf<W> &hz, const Vf<W> &hx_km, const Vf<W> &hy_km,
                                                const Vf<W> &hx_jm, const Vf<W> &hz_jm, float hy_im0, float hz_im0,
@@ -324,9 +322,9 @@ __device__ __forceinline__ void stream_e_group(Vf<W> &ex, Vf<W> &ey, Vf<W> &ez, 
             cx = c.x; cy = c.y; cz = c.z;
         }
         if (sp) {
-            cx -= dx * ldf1<COH>(sp + ij0 + e);
-            cy -= dx * ldf1<COH>(sp + nxy + ij0 + e);
-            cz -= dx * ldf1<COH>(sp + 2 * nxy + ij0 + e);
+            cx -= dx * sp[ij0 + e];
+            cy -= dx * sp[nxy + ij0 + e];
+            cz -= dx * sp[2 * nxy + ij0 + e];
         }
         ex.v[e] = c0.v[e] * ex.v[e] + b0.v[e] * cx;
         ey.v[e] = c1.v[e] * ey.v[e] + b1.v[e] * cy;
@@ -336,7 +334,7 @@ __device__ __forceinline__ void stream_e_group(Vf<W> &ex, Vf<W> &ey, Vf<W> &ez, 
 
 // H_new of one group (same roles as stream_e_group); ey_ipw, ez_ipw: new Ey,
 // Ez at x = i0 + W
-template <int W, bool X, bool EDGE, bool CPML, bool COH>
+template <int W, bool X, bool EDGE, bool CPML>
 __device__ __forceinline__ void stream_h_group(Vf<W> &nhx, Vf<W> &nhy, Vf<W> &nhz, const Vf<W> &ex, const Vf<W> &ey,
                                                const Vf<W> &exm, const Vf<W> &eym, const Vf<W> &ezm,
                                                const Vf<W> &ex_jp, const Vf<W> &ez_jp, float ey_ipw, float ez_ipw,
@@ -368,9 +366,9 @@ __device__ __forceinline__ void stream_h_group(Vf<W> &nhx, Vf<W> &nhy, Vf<W> &nh
             cx = c.x; cy = c.y; cz = c.z;
         }
         if (sp) {
-            cx += dx * ldf1<COH>(sp + 3 * nxy + ij0 + e);
-            cy += dx * ldf1<COH>(sp + 4 * nxy + ij0 + e);
-            cz += dx * ldf1<COH>(sp + 5 * nxy + ij0 + e);
+            cx += dx * sp[3 * nxy + ij0 + e];
+            cy += dx * sp[4 * nxy + ij0 + e];
+            cz += dx * sp[5 * nxy + ij0 + e];
         }
         nhx.v[e] = nhx.v[e] - hb * cx;
         nhy.v[e] = nhy.v[e] - hb * cy;
@@ -398,7 +396,7 @@ __device__ __forceinline__ void stream_plane_barrier() { asm volatile("bar.sync 
 //
 // TPC > 0: the staged rows a.ty + 1 known at compile time (the per-step kernel
 // is instantiated for 2..8; shared-memory offsets then fold into constants).
-template <bool CPML, bool LOSSY, bool COH = false, int TPC = 0>
+template <bool CPML, bool LOSSY, int TPC = 0>
 __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTile tl, float *sm)
 {
     constexpr int S = kStreamStages;
@@ -479,8 +477,8 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
             if (!CPML || it > n) return;
             const int k = tl.k0 + it;
             if (!yz_plane(k) && !yz_plane(k - 1)) return;
-            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<4, 0, COH>(yze, a, i0, j, k, ij0, nxy);
-            if (own && it >= 1) stream_yzpsi_load<4, 2, COH>(yzh, a, i0, j, k - 1, ij0, nxy);
+            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<4, 0>(yze, a, i0, j, k, ij0, nxy);
+            if (own && it >= 1) stream_yzpsi_load<4, 2>(yzh, a, i0, j, k - 1, ij0, nxy);
         };
         load_yz(0);
         XPsi<4> xnone;                               // interior quads hold no x-slab cell
@@ -527,16 +525,16 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
                 }
                 const float *sp = a.src.n ? src_plane(a.src, k) : nullptr;
                 if (!CPML)
-                    stream_e_group<4, false, true, false, LOSSY, COH>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm,
+                    stream_e_group<4, false, true, false, LOSSY>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm,
                                                                       hy_im0, hz_im0, b0, b1, b2, c0, c1, c2, xnone,
                                                                       yze, ptab, a, i0, sp, ij0, nxy, dx, div);
                 else if (!yz_plane(k))
-                    stream_e_group<4, false, false, false, LOSSY, COH>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm,
+                    stream_e_group<4, false, false, false, LOSSY>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm,
                                                                        hz_jm, hy_im0, hz_im0, b0, b1, b2, c0, c1, c2,
                                                                        xnone, yze, ptab, a, i0, sp, ij0, nxy, dx,
                                                                        div);
                 else
-                    stream_e_group<4, false, false, true, LOSSY, COH>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm,
+                    stream_e_group<4, false, false, true, LOSSY>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm,
                                                                       hy_im0, hz_im0, b0, b1, b2, c0, c1, c2, xnone,
                                                                       yze, ptab, a, i0, sp, ij0, nxy, dx, div);
             }
@@ -568,15 +566,15 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
                 Vf<4> nhx = hxm, nhy = hym, nhz = hzm;
                 const float *sp = a.src.n ? src_plane(a.src, km) : nullptr;
                 if (!CPML)
-                    stream_h_group<4, false, true, false, COH>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
+                    stream_h_group<4, false, true, false>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
                                                                ey_ipw, ez_ipw, xnone, yzh, ptab, a, i0, sp, ij0, nxy,
                                                                dx, div, hb);
                 else if (!yz_plane(km))
-                    stream_h_group<4, false, false, false, COH>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
+                    stream_h_group<4, false, false, false>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
                                                                 ey_ipw, ez_ipw, xnone, yzh, ptab, a, i0, sp, ij0, nxy,
                                                                 dx, div, hb);
                 else
-                    stream_h_group<4, false, false, true, COH>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
+                    stream_h_group<4, false, false, true>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp,
                                                                ey_ipw, ez_ipw, xnone, yzh, ptab, a, i0, sp, ij0, nxy,
                                                                dx, div, hb);
                 const sidx_t g = ij0 + nxy * (sidx_t)km;
@@ -667,8 +665,8 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
             if (it > n) return;
             const int k = tl.k0 + it;
             if (!yz_plane(k) && !yz_plane(k - 1)) return;
-            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<1, 0, COH>(yze, a, i, j, k, ij, nxy, ptab);
-            if (own && it >= 1) stream_yzpsi_load<1, 2, COH>(yzh, a, i, j, k - 1, ij, nxy, ptab);
+            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<1, 0>(yze, a, i, j, k, ij, nxy, ptab);
+            if (own && it >= 1) stream_yzpsi_load<1, 2>(yzh, a, i, j, k - 1, ij, nxy, ptab);
         };
         load_yz(0);
 
@@ -719,7 +717,7 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
                     c2.v[0] = stg(s, 11, r)[i];
                 }
                 const float *sp = a.src.n ? src_plane(a.src, k) : nullptr;
-                stream_e_group<1, true, true, true, LOSSY, COH>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm, hy_im0,
+                stream_e_group<1, true, true, true, LOSSY>(ex, ey, ez, hx, hy, hz, hxm, hym, hx_jm, hz_jm, hy_im0,
                                                                 hz_im0, b0, b1, b2, c0, c1, c2, xse, yze, ptab, a, i,
                                                                 sp, ij, nxy, dx, div);
             }
@@ -751,7 +749,7 @@ __device__ __forceinline__ void stream_tile(const StreamArgs &a, const StreamTil
                 const float ez_ipw = i < nx - 1 ? esp(b, 2, r)[i + 1] : 0.f;
                 Vf<1> nhx = hxm, nhy = hym, nhz = hzm;
                 const float *sp = a.src.n ? src_plane(a.src, km) : nullptr;
-                stream_h_group<1, true, true, true, COH>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp, ey_ipw,
+                stream_h_group<1, true, true, true>(nhx, nhy, nhz, ex, ey, exm, eym, ezm, ex_jp, ez_jp, ey_ipw,
                                                          ez_ipw, xsh, yzh, ptab, a, i, sp, ij, nxy, dx, div, hb);
                 const sidx_t g = ij + nxy * (sidx_t)km;
                 a.f_out[3][g] = nhx.v[0];

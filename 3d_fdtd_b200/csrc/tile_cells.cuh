@@ -292,9 +292,9 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                         float cy = (t.hx.v[x] - hp[0].v[x]) - (t.hz.v[x] - hzi);
                         float cz = (t.hy.v[x] - hyi) - (t.hx.v[x] - t.hxj.v[x]);
                         if (sp) {
-                            cx -= dx * __ldg(sp + ij0 + x);
-                            cy -= dx * __ldg(sp + nxy + ij0 + x);
-                            cz -= dx * __ldg(sp + 2 * nxy + ij0 + x);
+                            cx -= dx * sp[ij0 + x];
+                            cy -= dx * sp[nxy + ij0 + x];
+                            cz -= dx * sp[2 * nxy + ij0 + x];
                         }
                         e[0].v[x] = t.c.v[x] * e[0].v[x] + t.b.v[x] * cx;
                         e[1].v[x] = t.c.v[x] * e[1].v[x] + t.b.v[x] * cy;
@@ -321,9 +321,9 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                             float cy = (e[0].v[x] - ep[0].v[x]) - (ezi - ep[2].v[x]);
                             float cz = (eyi - ep[1].v[x]) - (exj.v[x] - ep[0].v[x]);
                             if (sph) {
-                                cx += dx * __ldg(sph + 3 * nxy + ij0 + x);
-                                cy += dx * __ldg(sph + 4 * nxy + ij0 + x);
-                                cz += dx * __ldg(sph + 5 * nxy + ij0 + x);
+                                cx += dx * sph[3 * nxy + ij0 + x];
+                                cy += dx * sph[4 * nxy + ij0 + x];
+                                cz += dx * sph[5 * nxy + ij0 + x];
                             }
                             h[0].v[x] = hp[0].v[x] - hb * cx;
                             h[1].v[x] = hp[1].v[x] - hb * cy;
@@ -355,13 +355,13 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                 p.pxy = fillv<4>(0.f); p.pzy = p.pxy; p.pxz = p.pxy; p.pyz = p.pxy;
                 if (Y && p.sj >= 0) {
                     const sidx_t sy = (sidx_t)i0 + (sidx_t)nx * (sidx_t)(p.sj + 2 * L * k);
-                    p.pxy = ldf<4, false>(a.psi_in[1][A0] + sy);
-                    p.pzy = ldf<4, false>(a.psi_in[1][A0 + 1] + sy);
+                    p.pxy = ldv_rw<4>(a.psi_in[1][A0] + sy);
+                    p.pzy = ldv_rw<4>(a.psi_in[1][A0 + 1] + sy);
                 }
                 if (Z && p.sk >= 0) {
                     const sidx_t sz = ij0 + nxy * (sidx_t)p.sk;
-                    p.pxz = ldf<4, false>(a.psi_in[2][A0] + sz);
-                    p.pyz = ldf<4, false>(a.psi_in[2][A0 + 1] + sz);
+                    p.pxz = ldv_rw<4>(a.psi_in[2][A0] + sz);
+                    p.pyz = ldv_rw<4>(a.psi_in[2][A0 + 1] + sz);
                 }
                 if (!Y) p.sj = -1;
                 if (!Z) p.sk = -1;
@@ -385,7 +385,7 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                     staged(s, t, e);
                     if (row_upd && k <= nz - 2) {
                         const float *sp = a.src.n ? src_plane(a.src, k) : nullptr;
-                        stream_e_group<4, false, false, true, LOSSY, false>(
+                        stream_e_group<4, false, false, true, LOSSY>(
                             e[0], e[1], e[2], t.hx, t.hy, t.hz, hp[0], hp[1], t.hxj, t.hzj, t.hyi, t.hzi, t.b, t.b,
                             t.b, t.c, t.c, t.c, xnone, yze, ptab, a, i0, sp, ij0, nxy, dx, div);
                     }
@@ -402,7 +402,7 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                         const Vf<4> ep0 = lds4(pe), ep1 = lds4(pe + A), ep2 = lds4(pe + 2 * A);
                         const Vf<4> exj = lds4(pe + row_st), ezj = lds4(pe + row_st + 2 * A);
                         const float *sp = a.src.n ? src_plane(a.src, km) : nullptr;
-                        stream_h_group<4, false, false, true, false>(hp[0], hp[1], hp[2], e[0], e[1], ep0, ep1, ep2, exj,
+                        stream_h_group<4, false, false, true>(hp[0], hp[1], hp[2], e[0], e[1], ep0, ep1, ep2, exj,
                                                                      ezj, pe[A + 4], pe[2 * A + 4], xnone,
                                                                      yzh, ptab, a, i0, sp, ij0, nxy, dx, div, hb);
                         store3(3, km, hp);
@@ -498,8 +498,8 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
             if (it > n) return;
             const int k = tl.k0 + it;
             if (!yz_plane(k) && !yz_plane(k - 1)) return;
-            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<1, 0, false>(yze, a, i, j, k, ij, nxy, ptab);
-            if (own && it >= 1) stream_yzpsi_load<1, 2, false>(yzh, a, i, j, k - 1, ij, nxy, ptab);
+            if (act && row_upd && k <= nz - 2) stream_yzpsi_load<1, 0>(yze, a, i, j, k, ij, nxy, ptab);
+            if (own && it >= 1) stream_yzpsi_load<1, 2>(yzh, a, i, j, k - 1, ij, nxy, ptab);
         };
         load_yz(0);
         Vf<1> hxm = fillv<1>(0.f), hym = hxm, hzm = hxm;           // old H of the cell in the plane below
@@ -546,7 +546,7 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                 b.v[0] = rec[6 * A];
                 if (LOSSY) c.v[0] = rec[7 * A];
                 const float *sp = a.src.n ? src_plane(a.src, k) : nullptr;
-                stream_e_group<1, true, true, true, LOSSY, false>(ex, ey, ez, hx, hy, hz, hxm, hym, hxj, hzj, hyi, hzi,
+                stream_e_group<1, true, true, true, LOSSY>(ex, ey, ez, hx, hy, hz, hxm, hym, hxj, hzj, hyi, hzi,
                                                                   b, b, b, c, c, c, xse, yze, ptab, a, i, sp, ij, nxy,
                                                                   dx, div);
             }
@@ -573,7 +573,7 @@ __device__ __forceinline__ void yee_tile(const StreamArgs &a, const TileMaps *ma
                 exj.v[0] = pe[row_st];
                 ezj.v[0] = pe[row_st + 2 * A];
                 const float *sp = a.src.n ? src_plane(a.src, km) : nullptr;
-                stream_h_group<1, true, true, true, false>(hxm, hym, hzm, ex, ey, exm, eym, ezm, exj, ezj, pe[A + 1], pe[2 * A + 1],
+                stream_h_group<1, true, true, true>(hxm, hym, hzm, ex, ey, exm, eym, ezm, exj, ezj, pe[A + 1], pe[2 * A + 1],
                                                            xsh, yzh, ptab, a, i, sp, ij, nxy, dx, div, hb);
                 const sidx_t g = ij + nxy * (sidx_t)km;
                 a.f_out[3][g] = hxm.v[0];

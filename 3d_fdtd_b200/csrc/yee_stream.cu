@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kStreamMaxThreads, 1) k_yee_stream(StreamArgs 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) float sm[];
-    stream_tile<CPML, LOSSY, false, TPC>(a, a.tiles[blockIdx.x], sm);
+    stream_tile<CPML, LOSSY, TPC>(a, a.tiles[blockIdx.x], sm);
 }
 
 using StreamKernel = void (*)(StreamArgs);

@@ -115,7 +115,7 @@ template <bool CPML, bool LOSSY, int TPC>
 __device__ __forceinline__ void sweep_tile(int idx, int t, float *sm)
 {
     const StreamArgs &sa = c_sweep_args[idx];
-    stream_tile<CPML, LOSSY, true, TPC>(sa, sa.tiles[t], sm);
+    stream_tile<CPML, LOSSY, TPC>(sa, sa.tiles[t], sm);
 }
 
 // TPC: the staged rows of every grid's tiles when they agree and are one of

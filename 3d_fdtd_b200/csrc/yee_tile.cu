@@ -19,8 +19,8 @@
 //  - all columns are cut at the same planes, in one or two waves of blocks: tiles
 //    that run side by side read a shared halo row from DRAM once (kInStep below).
 // Per step, before (three coefficients, cp.async) and now: 200x160x400 with CPML 189
-// and 158 us (5.05 TB/s of algorithmic bytes), with PEC 144 and 115 us; 384x256x384
-// CPML 792 and 414; 256x128x128 CPML 77 and 67; 96x80x64 CPML, conductivity 45 and
+// and 160 us (5.02 TB/s of algorithmic bytes), with PEC 144 and 115 us; 384x256x384
+// CPML 792 and 411; 256x128x128 CPML 77 and 69; 96x80x64 CPML, conductivity 45 and
 // 14 us.  Two blocks an SM (96 registers) spill with CPML and gave nothing without.
 #include "tile_cells.cuh"
 #include "plane_ops.cuh"

@@ -123,25 +123,25 @@ __device__ __forceinline__ void wave_cells(const FlatArgs &a, const Plan4 &p, bo
     bool live;
     if (p.L == 0) {
         locate<0>(p.zs, a.nx / 4, a.ny, s, k - 1, g, j, kk, live);
-        if (efield) e_cells<4, 0, LOSSY, true>(a, g, j, kk, live, ls);
-        else h_cells<4, 0, true>(a, g, j, kk, live, ls);
+        if (efield) e_cells<4, 0, LOSSY>(a, g, j, kk, live, ls);
+        else h_cells<4, 0>(a, g, j, kk, live, ls);
     } else if (k < p.L || k >= a.nz - p.L) {
         const int by = k < p.L ? k - 1 : (p.L - 1) + (k - (a.nz - p.L));
         locate<0>(p.zs, a.nx / 2, a.ny, s, by, g, j, kk, live);
-        if (efield) e_cells<2, 7, LOSSY, true>(a, g, j, kk, live, ls);
-        else h_cells<2, 7, true>(a, g, j, kk, live, ls);
+        if (efield) e_cells<2, 7, LOSSY>(a, g, j, kk, live, ls);
+        else h_cells<2, 7>(a, g, j, kk, live, ls);
     } else if (lb < p.nb_box) {
         locate<1>(p.box, a.nx / 4, a.ny, s, k - p.L, g, j, kk, live);
-        if (efield) e_cells<4, 0, LOSSY, true>(a, g, j, kk, live, ls);
-        else h_cells<4, 0, true>(a, g, j, kk, live, ls);
+        if (efield) e_cells<4, 0, LOSSY>(a, g, j, kk, live, ls);
+        else h_cells<4, 0>(a, g, j, kk, live, ls);
     } else if (lb < p.nb_box + p.nb_y) {
         locate<3>(p.yrows, a.nx / 2, a.ny, s - p.nb_box * kBlock4, k - p.L, g, j, kk, live);
-        if (efield) e_cells<2, 2, LOSSY, true>(a, g, j, kk, live, ls);
-        else h_cells<2, 2, true>(a, g, j, kk, live, ls);
+        if (efield) e_cells<2, 2, LOSSY>(a, g, j, kk, live, ls);
+        else h_cells<2, 2>(a, g, j, kk, live, ls);
     } else {
         locate<4>(p.xcols, a.nx / 2, a.ny, s - (p.nb_box + p.nb_y) * kBlock4, k - p.L, g, j, kk, live);
-        if (efield) e_cells<2, 3, LOSSY, true>(a, g, j, kk, live, ls);
-        else h_cells<2, 3, true>(a, g, j, kk, live, ls);
+        if (efield) e_cells<2, 3, LOSSY>(a, g, j, kk, live, ls);
+        else h_cells<2, 3>(a, g, j, kk, live, ls);
     }
 }
 

@@ -40,3 +40,23 @@ def test_split_step_kernels_wait_first():
         first = [s.strip() for s in b.split(";")]
         first = [s for s in first if s and not s.startswith("using ")]
         assert first[0] == "after_previous()", (k, first[0])
+
+
+def test_read_only_loads_take_only_what_no_step_writes():
+    # the read-only path (__ldg) is for data that nothing writes while the kernel lives, and a
+    # kernel started programmatically lives while the launch before it still writes fields,
+    # auxiliaries and source planes: coefficients and profiles only
+    constant = re.compile(r"a\.(prof\[[^\]]+\]\[[^\]]+\]|c[ab]\[[^\]]+\]) \+ ")
+    seen = 0
+    for name in ("yee_tile.cu", "tile_cells.cuh", "yee_stream.cu", "stream_cells.cuh", "yee_flat4.cu", "flat4_cells.cuh",
+                 "yee_flat.cu", "yee_split.cu", "yee_wave.cu", "yee_sweep.cu", "aux_kernels.cu", "plane_ops.cuh"):
+        text = source(name)
+        if name == "flat4_cells.cuh":   # the vector form of the load itself
+            start = text.index("Vf<W> ldv(")
+            text = text.replace(body(text, start), "", 1)
+            text = text.replace("Vf<W> ldv(", "", 1)
+        for arg in re.findall(r"(?:__ldg|\bldv<\w+>)\(([^;]*?)\)[,;\s]", text):
+            assert constant.match(arg), (name, arg)
+            seen += 1
+        assert "ld.global.nc" not in text
+    assert seen > 10
