@@ -244,13 +244,14 @@ bool stream_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, StreamPlan 
     return true;
 }
 
+// (one limit for every plan, as tile_configure)
 bool stream_configure(size_t smem, int threads)
 {
     if (smem > kStreamSmemBudget) return false;
     for (int v = 0; v < 4; v++)
         for (int tp = 1; tp <= 8; tp++) {   // 1: the run-time-rows kernel
             const void *f = (const void *)stream_kernel((v & 2) != 0, (v & 1) != 0, tp);
-            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmemBudget) != cudaSuccess)
                 return false;
             cudaFuncAttributes at{};
             if (cudaFuncGetAttributes(&at, f) != cudaSuccess || at.maxThreadsPerBlock < threads) return false;

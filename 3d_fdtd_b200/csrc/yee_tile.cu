@@ -405,13 +405,15 @@ bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out
     return true;
 }
 
+// (the limit is the kernel's, not a grid's: always the same one, so that no plan takes
+// it from the grids prepared before; a launch names its own size)
 bool tile_configure(size_t smem, int threads)
 {
     if (smem > kStreamSmemBudget) return false;
     for (int v = 0; v < 4; v++) {
         const void *f = (const void *)tile_kernel((v & 2) != 0, (v & 1) != 0);
         cudaFuncAttributes at{};
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmemBudget) != cudaSuccess ||
             cudaFuncGetAttributes(&at, f) != cudaSuccess || at.maxThreadsPerBlock < threads)
             return false;
     }
