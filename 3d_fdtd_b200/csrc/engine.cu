@@ -731,6 +731,7 @@ static bool stream_prepare(Grid *g)
         return false;
     }
     CK(cudaStreamSynchronize(g->st));
+    std::fill(g->splan_key, g->splan_key + 6, -1);   // unset until the new list is in place
     dfree(g->d_tiles);
     if (!dalloc(&g->d_tiles, p.tiles.size() * sizeof(StreamTile), g->st, false)) return false;
     CK(cudaMemcpyAsync(g->d_tiles, p.tiles.data(), p.tiles.size() * sizeof(StreamTile), cudaMemcpyHostToDevice, g->st));
@@ -753,31 +754,39 @@ static bool tile_prepare(Grid *g)
         for (int m = 0; m < 6; m++) arrays[2 + 6 * s + m] = g->f[s][m];
     const bool same_plan = g->d_boxes && std::equal(key, key + 6, g->tplan_key);
     if (same_plan && std::equal(arrays, arrays + 14, g->maps_of)) return true;
-    TilePlan p;
-    if (!tile_plan(g->nx, g->ny, g->nz, L, g->sig_e, nsm, &p)) {
-        set_error(FDTD_ERR_UNSUPPORTED, "streaming Yee kernel: no tile plan for grid %dx%dx%d", g->nx, g->ny, g->nz);
-        return false;
+    // What fails half-way leaves its key unset, so that no later call takes tiles,
+    // plan and descriptors of different settings together.
+    std::fill(g->maps_of, g->maps_of + 14, nullptr);
+    if (!same_plan) {
+        TilePlan p;
+        if (!tile_plan(g->nx, g->ny, g->nz, L, g->sig_e, nsm, &p)) {
+            set_error(FDTD_ERR_UNSUPPORTED, "streaming Yee kernel: no tile plan for grid %dx%dx%d", g->nx, g->ny, g->nz);
+            return false;
+        }
+        if (!tile_configure(p.smem, p.threads)) {
+            set_error(FDTD_ERR_CUDA,
+                      "streaming Yee kernel: blocks of %d threads with %zu bytes of shared memory cannot launch",
+                      p.threads, p.smem);
+            return false;
+        }
+        CK(cudaStreamSynchronize(g->st));
+        std::fill(g->tplan_key, g->tplan_key + 6, -1);
+        dfree(g->d_boxes);
+        const size_t bytes = p.tiles.size() * sizeof(TileBox);
+        if (!dalloc(&g->d_boxes, bytes, g->st, false)) return false;
+        CK(cudaMemcpyAsync(g->d_boxes, p.tiles.data(), bytes, cudaMemcpyHostToDevice, g->st));
+        g->tplan = std::move(p);
+        std::copy(key, key + 6, g->tplan_key);
     }
-    if (!tile_configure(p.smem, p.threads)) {
-        set_error(FDTD_ERR_CUDA, "streaming Yee kernel: blocks of %d threads with %zu bytes of shared memory cannot launch",
-                  p.threads, p.smem);
-        return false;
-    }
-    CK(cudaStreamSynchronize(g->st));
-    dfree(g->d_boxes);
-    if (!dalloc(&g->d_boxes, p.tiles.size() * sizeof(TileBox), g->st, false)) return false;
-    CK(cudaMemcpyAsync(g->d_boxes, p.tiles.data(), p.tiles.size() * sizeof(TileBox), cudaMemcpyHostToDevice, g->st));
     TileMaps maps[2];
     for (int s = 0; s < 2; s++)
         if (!tile_make_maps(&maps[s], (const float *const *)g->f[s], g->cb[0], g->sig_e ? g->ca[0] : nullptr, g->nx,
-                            g->ny, g->nz, p)) {
+                            g->ny, g->nz, g->tplan)) {
             set_error(FDTD_ERR_CUDA, "streaming Yee kernel: TMA descriptors of a %dx%dx%d grid", g->nx, g->ny, g->nz);
             return false;
         }
     if (!dalloc(&g->d_maps, sizeof maps, g->st, false)) return false;
     CK(cudaMemcpyAsync(g->d_maps, maps, sizeof maps, cudaMemcpyHostToDevice, g->st));
-    g->tplan = std::move(p);
-    std::copy(key, key + 6, g->tplan_key);
     std::copy(arrays, arrays + 14, g->maps_of);
     g->version++;
     return true;
