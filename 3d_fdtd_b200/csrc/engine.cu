@@ -692,8 +692,15 @@ static bool fast32_path(const Grid *g)
 // three (yee_stream.cu, 60 B).
 static bool tile_path(const Grid *g)
 {
-    return fast32_path(g) && (g->yee_variant == FDTD_YEE_STREAM || g->yee_variant == FDTD_YEE_AUTO) && g->mat_iso &&
-           tile_supported(g->nx, g->ny, g->nz, g->sig_e, g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0);
+    if (!fast32_path(g) || !(g->yee_variant == FDTD_YEE_STREAM || g->yee_variant == FDTD_YEE_AUTO) || !g->mat_iso)
+        return false;
+    // a search over column cuts: once a setting, since every step asks several times
+    const int key[2] = {g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0, g->sig_e ? 1 : 0};
+    if (!std::equal(key, key + 2, g->tile_key)) {
+        g->tile_ok = tma_available() && tile_supported(g->nx, g->ny, g->nz, g->sig_e, key[0]);
+        std::copy(key, key + 2, g->tile_key);
+    }
+    return g->tile_ok;
 }
 
 static bool stream_path(const Grid *g)

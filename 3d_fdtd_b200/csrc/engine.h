@@ -136,6 +136,8 @@ struct Grid {
     TileMaps *d_maps = nullptr;      // two: set 0, set 1 as input
     const void *maps_of[14] = {};    // the arrays they describe
     int tplan_key[6] = {-1, -1, -1, -1, -1, -1};
+    mutable int tile_key[2] = {-1, -1};   // L, lossy that tile_ok is for
+    mutable bool tile_ok = false;         // the kernel takes grids of this shape
     double2 *d_sums = nullptr;       // a chain's overlap sums, two steps (StepChain)
     size_t sums_cap = 0;
     float *d_src2 = nullptr;         // the scheduled source's plane on odd steps of a chain

@@ -399,6 +399,8 @@ struct FusedMaps {
     CUtensorMap ca[3];
 };
 int fused_tma_supported(int nx, int ny, int nz);
+// the driver encodes TMA descriptors
+bool tma_available();
 // descriptor of an nx x ny x nz float array, boxes of box_x x box_y cells of one plane
 bool tma_encode_3d(CUtensorMap *m, const float *base, int nx, int ny, int nz, int box_x, int box_y);
 bool fused_make_maps(FusedMaps *m, const float *const f[6], const float *const cb[3], const float *const ca[3],

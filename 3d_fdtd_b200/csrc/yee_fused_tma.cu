@@ -526,6 +526,8 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
     return fn;
 }
 
+bool tma_available() { return encode_fn() != nullptr; }
+
 constexpr int kTY = 8;   // tile height (rows per thread = kTY / 8)
 
 int fused_tma_supported(int nx, int ny, int nz) { return nx % 4 == 0 && nx >= 8 && ny >= 4 && nz >= 4 && encode_fn(); }
