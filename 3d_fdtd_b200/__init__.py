@@ -193,6 +193,7 @@ SIGNATURES = {
     "fdtd_sweep_run": (i, [C.POINTER(T), i, d, ip, i, i, d]),
     "fdtd_sweep_barrier_selftest": (i, [d]),
     "fdtd_stream_plan": (i, [i, i, i, i, i, i, ip, i, ip, ip, C.POINTER(C.c_longlong)]),
+    "fdtd_tile_plan": (i, [i, i, i, i, i, i, ip, i, ip, ip, C.POINTER(C.c_longlong)]),
     "fdtd_mode_overlap_plane_noalloc": (i, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, i, i, i, i, i,
                                             C.c_void_p, i, i, d, i, d, C.c_void_p, C.c_void_p]),
 }

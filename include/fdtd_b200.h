@@ -282,6 +282,12 @@ int fdtd_wave_schedule(int nx, int ny, int nz, int cpml_cells, int steps, int sw
  * when the grid cannot use the kernel or on invalid input. */
 int fdtd_stream_plan(int nx, int ny, int nz, int cpml_cells, int lossy, int nsm, int *tiles, int cap, int *ty,
                      int *threads, long long *smem_bytes);
+/* The same for grids whose coefficients agree on a cell's components (the default
+ * step).  6 ints per tile: first owned quad (4 x cells), one past the last, first
+ * owned row, owned rows, first owned plane, one past the last; and the rows a block
+ * stages (one more than it owns at most). */
+int fdtd_tile_plan(int nx, int ny, int nz, int cpml_cells, int lossy, int nsm, int *tiles, int cap, int *staged_rows,
+                   int *threads, long long *smem_bytes);
 /* CPML of `thickness` cells on every face, polynomial grading `order`;
  * sigma_max <= 0 selects 0.8 (order+1)/disc; kappa_max >= 1; alpha_max >= 0.
  * Profiles depend on delta_t and are rebuilt when the step size changes.
