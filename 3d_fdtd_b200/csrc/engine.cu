@@ -697,7 +697,14 @@ static bool tile_path(const Grid *g)
     // a search over column cuts: once a setting, since every step asks several times
     const int key[2] = {g->boundary == FDTD_BOUNDARY_CPML ? g->L : 0, g->sig_e ? 1 : 0};
     if (!std::equal(key, key + 2, g->tile_key)) {
-        g->tile_ok = tma_available() && tile_supported(g->nx, g->ny, g->nz, g->sig_e, key[0]);
+        // Rows too long for the three-coefficient kernel (over about 750 cells) on few
+        // cells are mostly slabs in tiles of a few planes, while the two-kernel step finds
+        // what it reads twice in L2.  With a CPML, tile and two-kernel step: 1000x40x40
+        // 43 and 33 us, 1900x24x24 24 and 19, 1000x50x50 38 and 32, 1000x64x50 66 and 64;
+        // 1000x60x64 56 and 60, 900x70x70 73 and 85, 1000x100x100 148 and 176.  (Of larger
+        // ones that are mostly slabs up to 5 % slower in tiles: 1000x24x400 194 and 185.)
+        const bool small_wide = key[0] > 0 && g->n < 3500000 && !stream_supported(g->nx, g->ny, g->nz, g->sig_e, key[0]);
+        g->tile_ok = !small_wide && tma_available() && tile_supported(g->nx, g->ny, g->nz, g->sig_e, key[0]);
         std::copy(key, key + 2, g->tile_key);
     }
     return g->tile_ok;
