@@ -61,9 +61,11 @@ def candidates(n: int = 64, seed: int = 2, ncontrol: int = 20, steps_scale: floa
     return out
 
 
-def algorithmic_bytes(nx: int, ny: int, nz: int, L: int) -> int:
-    """Per time step: 60 B per cell + 32 B per (cell, CPML axis), FP32."""
-    return 60 * nx * ny * nz + 32 * (2 * L * ny * nz + nx * 2 * L * nz + nx * ny * 2 * L)
+def algorithmic_bytes(nx: int, ny: int, nz: int, L: int, coefficients: int = 3) -> int:
+    """Per time step, FP32: 48 B per cell (6 field components read and written), 4 B per
+    E coefficient read (1 where a cell's three are equal and the kernel reads one), and
+    32 B per (cell, CPML axis)."""
+    return (48 + 4 * coefficients) * nx * ny * nz + 32 * (2 * L * ny * nz + nx * 2 * L * nz + nx * ny * 2 * L)
 
 
 def source_tables(T: int, dt: float):
@@ -216,6 +218,8 @@ def sweep(fd, cands: list[dict], slots: int = 4, variant: int | None = None, ret
     amplitudes = {}
     cell_steps = 0
     nbytes = 0
+    # candidates come from the rasterisers, which write a cell's three alike
+    coefficients = 3 if variant in (fd.YEE_FLAT4, fd.YEE_FUSED, fd.YEE_WAVE) else 1
     t0 = time.perf_counter()
     for slot in pool:
         if not queue:
@@ -231,7 +235,7 @@ def sweep(fd, cands: list[dict], slots: int = 4, variant: int | None = None, ret
         results[c["index"]] = (np.abs(t) ** 2).tolist()
         nx, ny, nz = slot.shape
         cell_steps += nx * ny * nz * c["steps"]
-        nbytes += algorithmic_bytes(nx, ny, nz, SPEC["cpml"]) * c["steps"]
+        nbytes += algorithmic_bytes(nx, ny, nz, SPEC["cpml"], coefficients) * c["steps"]
         if queue:
             prepare(slot, queue.pop(0))
             slot.start()
@@ -316,7 +320,7 @@ def sweep_persistent(fd, cands: list[dict], group: int = 8, steps_per_launch: in
             results[c["index"]] = (np.abs(t) ** 2).tolist()
             nx, ny, nz = s.shape
             cell_steps += nx * ny * nz * c["steps"]
-            nbytes += algorithmic_bytes(nx, ny, nz, SPEC["cpml"]) * c["steps"]
+            nbytes += algorithmic_bytes(nx, ny, nz, SPEC["cpml"], 1) * c["steps"]
         for s in current:
             s.close()
         current = nxt
