@@ -287,14 +287,16 @@ def autotune_tiles(fd, cands: list[dict], steps: int = 128, steps_per_launch: in
 def sweep_persistent(fd, cands: list[dict], group: int = 8, steps_per_launch: int = 64,
                      shape: tuple[int, float] | None = None) -> dict:
     """Every candidate through fdtd_sweep_run: candidates sorted by step count,
-    `group` at a time advance together (of uneven lengths); the next group is set up on the host while the current one runs."""
+    `group` at a time advance together (of uneven lengths); the next group is set up on
+    the host while the current one runs.  `steps_per_launch` and `shape` (band rows,
+    tiles per SM) are fdtd_sweep_run's, for grids whose coefficients differ; the
+    rasterisers' do not, so nothing is timed to choose them."""
     if not cands:
         return dict(results={}, amplitudes={}, seconds=0.0, cell_steps=0, bytes=0, shape=None, tuning={})
     order = sorted(cands, key=lambda c: c["steps"])
     groups = [order[i:i + group] for i in range(0, len(order), group)]
-    tuning = {}
     if shape is None:
-        shape, tuning = autotune_tiles(fd, groups[-1][:group])
+        shape = (0, 2.0)
     results, amplitudes = {}, {}
     cell_steps = nbytes = 0
     t0 = time.perf_counter()
@@ -326,7 +328,7 @@ def sweep_persistent(fd, cands: list[dict], group: int = 8, steps_per_launch: in
         current = nxt
     seconds = time.perf_counter() - t0
     return dict(results=results, amplitudes=amplitudes, seconds=seconds, cell_steps=cell_steps, bytes=nbytes,
-                shape=list(shape), tuning={f"{k[0]}x{k[1]}": v for k, v in tuning.items()})
+                shape=list(shape), tuning={})
 
 
 def main():
@@ -366,7 +368,7 @@ def main():
         line = dict(metric="candidate sweep Yee Mcell-updates/s", value=cell_steps / seconds / 1e6,
                     unit="Mcell-updates/s", n_gpus=ranks.world, candidates=len(cands), seconds=seconds,
                     hbm_frac=nbytes / seconds / 1e9 / (peak * ranks.world), slots=args.slots,
-                    mode=args.mode, group=args.group, tile_shape=r.get("shape"),
+                    mode=args.mode, group=args.group,
                     variant=r["variant"], tuning_ms_per_step=r["tuning"],
                     T_mean_1550=float(np.mean([t[5] for t in T])),
                     T_best_1550=float(np.max([t[5] for t in T])))

@@ -415,8 +415,8 @@ def our_arm(args, rank: int, world: int, local_rank: int) -> None:
     torch.cuda.synchronize()
     e2e_s = max_over_ranks(time.perf_counter() - t0)
     e2e = world * cells * args.time_steps * args.steps / e2e_s / 1e6
-    # candidate sweep (64-candidate taper family, seeded subset): grouped
-    # multi-grid launches with the tile-shape autotuner, host clock around it
+    # candidate sweep (64-candidate taper family, seeded subset) in one call, host
+    # clock around it
     sweep = None
     if rank == 0 and world == 1 and args.sweep_candidates > 0:
         batch = importlib.import_module("3d_fdtd_b200.batch")
@@ -426,7 +426,6 @@ def our_arm(args, rank: int, world: int, local_rank: int) -> None:
         sweep = {"candidates": len(cands), "of": "64-candidate taper family (seed 2), first candidates",
                  "value": r["cell_steps"] / r["seconds"] / 1e6, "unit": "Mcell-updates/s",
                  "hbm_frac": r["bytes"] / r["seconds"] / 1e9 / peak_gbs, "seconds": r["seconds"],
-                 "tile_shape": r["shape"], "autotune_ms_per_step": r["tuning"],
                  "launch": "one call; each candidate's steps in graphs on its own stream"}
     # FP32 against FP64: the same workload once on the engine's FP64 path (bit-exact
     # to the CPU restatement on CPML grids), outside every timed region

@@ -1,5 +1,6 @@
 """What a candidate sweep reports of itself, with the simulations left out: the bytes
-of the kernel its candidates take."""
+of the kernel its candidates take, and no time spent on choosing what does not act on
+them."""
 from __future__ import annotations
 
 import importlib
@@ -59,3 +60,14 @@ def test_sweep_bytes_are_the_kernels(engine, B):
     assert B.sweep_persistent(engine, cands, group=2, shape=(0, 2.0))["bytes"] == moved(cands, 52)
     assert B.sweep(engine, cands, slots=2, variant=engine.YEE_STREAM)["bytes"] == moved(cands, 52)
     assert B.sweep(engine, cands, slots=2, variant=engine.YEE_FLAT4)["bytes"] == moved(cands, 60)
+
+
+def test_sweep_times_no_tile_shapes(engine, B, monkeypatch):
+    # candidates come from the rasterisers: fdtd_sweep_run gives them streams of their own,
+    # which its tile shape does not touch
+    def tune(*a, **k):
+        raise AssertionError("tile shapes timed")
+
+    monkeypatch.setattr(B, "autotune_tiles", tune)
+    r = B.sweep_persistent(engine, B.candidates(2, seed=2), group=2)
+    assert sorted(r["results"]) == [0, 1] and r["tuning"] == {}
