@@ -228,7 +228,7 @@ struct MsKrylov {
     ulonglong2 *words;   // partials [value][block](re, im), then sums [value] kWordStride apart; zero at launch
     unsigned *bar;       // zero at launch
     int *err;
-    double2 *gram;       // K x K for each block, when it does not fit shared memory
+    double2 *gram;       // K x K, when it does not fit the blocks' shared memory
     unsigned long long wait_ns;
 };
 constexpr int kWordStride = 8;   // a sum's words on a cache line of their own: every block polls them
@@ -311,7 +311,7 @@ template <int EPT> __global__ void __launch_bounds__(kDotThreads) k_ms_krylov(Ms
     constexpr int R = EPT > 0 ? EPT : 1;
     double2 *wsum = dyn;                         // [warp][2K]: the warps' sums of a reduction
     double2 *sums = dyn + kDotWarps * 2 * K;     // [2K]: its result
-    double2 *G = a.gram ? a.gram + (size_t)blockIdx.x * K * K : sums + 2 * K;
+    double2 *G = a.gram ? a.gram : sums + 2 * K;   // <k_row, k_col> at [col][row]
     ulonglong2 *part = a.words, *total = a.words + (size_t)4 * K * kDotBlocks;
     double2 yr[R], qr[R];       // y and k_{i-1}
     unsigned nbar = 0, nred = 0;
@@ -383,21 +383,28 @@ template <int EPT> __global__ void __launch_bounds__(kDotThreads) k_ms_krylov(Ms
             if (l + 1 < i) warp_sum_to(wsum + warp * 2 * K + i + l, gs);
         }
         if (!reduce(2 * i - 1)) return;
-        for (int l = tid; l + 1 < i; l += kDotThreads) G[(size_t)(i - 1) * K + l] = sums[i + l];
+        // in device memory it is the grid's: block 0 writes it, the others take this step's
+        // row from their sums and the rows before from there, a grid barrier later
+        if (!a.gram || blockIdx.x == 0)
+            for (int l = tid; l + 1 < i; l += kDotThreads) G[(size_t)l * K + (i - 1)] = sums[i + l];
         __syncthreads();
+        auto gram = [&](int row, int col) {
+            if (!a.gram) return G[(size_t)col * K + row];
+            return row == i - 1 ? sums[i + col] : __ldcg(G + (size_t)col * K + row);
+        };
         // h from (I + strictly lower G) h = s, in place, by one warp
         if (warp == 0) {
             if (K <= 32) {
                 double2 h = lane < i ? sums[lane] : make_double2(0.0, 0.0);
                 for (int j = 0; j + 1 < i; j++) {
                     const double2 hj = make_double2(__shfl_sync(0xffffffffu, h.x, j), __shfl_sync(0xffffffffu, h.y, j));
-                    if (lane > j && lane < i) h = csub(h, cmul(hj, G[(size_t)lane * K + j]));
+                    if (lane > j && lane < i) h = csub(h, cmul(hj, gram(lane, j)));
                 }
                 if (lane < i) sums[lane] = h;
             } else {
                 for (int j = 0; j + 1 < i; j++) {
                     const double2 hj = sums[j];
-                    for (int k = j + 1 + lane; k < i; k += 32) sums[k] = csub(sums[k], cmul(hj, G[(size_t)k * K + j]));
+                    for (int k = j + 1 + lane; k < i; k += 32) sums[k] = csub(sums[k], cmul(hj, gram(k, j)));
                     __syncwarp();
                 }
             }
@@ -811,7 +818,7 @@ struct Solver {
                      o_done = slab.add<unsigned>(4), o_scal = slab.add<double2>((kv + 1) * (kv + 1) + 8),
                      o_y = slab.add<double2>(kv + 1), o_prev = slab.add<double2>(np * 2 * nn),
                      o_f = slab.add<double2>(6 * nn),
-                     o_gram = slab.add<double2>(gram_shared(kv - 1) ? 0 : kDotBlocks * (kv - 1) * (kv - 1));
+                     o_gram = slab.add<double2>(gram_shared(kv - 1) ? 0 : (kv - 1) * (kv - 1));
         MSK(cudaMalloc(&slab.p, slab.used));
         slab.at(o_ep, &ep); slab.at(o_mu, &mu); slab.at(o_pml, &pml); slab.at(o_iez, &iez); slab.at(o_imz, &imz);
         slab.at(o_is2, &is2); slab.at(o_psi, &psi); slab.at(o_basis, &basis); slab.at(o_tmp, &tmp);
