@@ -1396,30 +1396,34 @@ int fdtd_wait_selftest(double limit_seconds, double *elapsed_seconds)
         set_error(FDTD_ERR_ARG, "wait self-test limit %g s: must be in (0, 10]", limit_seconds);
         return FDTD_ERR_ARG;
     }
+    // the fused step's wait, the streaming tile's, the mode solver's
+    constexpr int kWaits = 3;
+    struct Status {
+        unsigned long long ns[kWaits];
+        int err[kWaits];
+        unsigned bar;
+    } h{}, *d = nullptr;
     cudaStream_t st = nullptr;
-    int *d_err = nullptr;
-    unsigned long long *d_el = nullptr;
-    int h_err = 0;
-    unsigned long long h_el = 0;
     bool ok = cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate") &&
-              cuda_ok(cudaMalloc(&d_err, sizeof(int)), "cudaMalloc") &&
-              cuda_ok(cudaMalloc(&d_el, sizeof(unsigned long long)), "cudaMalloc") &&
-              cuda_ok(cudaMemsetAsync(d_err, 0, sizeof(int), st), "cudaMemsetAsync");
+              cuda_ok(cudaMalloc(&d, sizeof h), "cudaMalloc") &&
+              cuda_ok(cudaMemsetAsync(d, 0, sizeof h, st), "cudaMemsetAsync");
     if (ok) {
-        launch_wait_selftest((unsigned long long)(limit_seconds * 1e9), d_err, d_el, st);
+        const unsigned long long limit = (unsigned long long)(limit_seconds * 1e9);
+        launch_wait_selftest(limit, &d->err[0], &d->ns[0], st);
+        launch_tile_wait_selftest(limit, &d->err[1], &d->ns[1], st);
+        launch_mode_wait_selftest(limit, &d->bar, &d->err[2], &d->ns[2], st);
         ok = cuda_ok(cudaGetLastError(), "wait self-test launch") &&
-             cuda_ok(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync") &&
-             cuda_ok(cudaMemcpyAsync(&h_el, d_el, sizeof(h_el), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync") &&
+             cuda_ok(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync") &&
              cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     }
-    if (d_err) cudaFree(d_err);
-    if (d_el) cudaFree(d_el);
+    if (d) cudaFree(d);
     if (st) cudaStreamDestroy(st);
     if (!ok) return fdtd_last_error();
-    if (elapsed_seconds) *elapsed_seconds = (double)h_el * 1e-9;
-    if (h_err) {
-        set_error(FDTD_ERR_TIMEOUT, "wait self-test: the bounded wait gave up after %.3f s as designed",
-                  (double)h_el * 1e-9);
+    const double longest = (double)*std::max_element(h.ns, h.ns + kWaits) * 1e-9;
+    if (elapsed_seconds) *elapsed_seconds = longest;
+    if (h.err[0] && h.err[1] && h.err[2]) {
+        set_error(FDTD_ERR_TIMEOUT, "wait self-test: the bounded waits gave up after %.3f s at most, as designed",
+                  longest);
         return FDTD_ERR_TIMEOUT;
     }
     set_error(FDTD_ERR_CUDA, "wait self-test: a wait on a barrier nothing arrives on completed");

@@ -407,6 +407,10 @@ bool fused_make_maps(FusedMaps *m, const float *const f[6], const float *const c
                      int nx, int ny, int nz);
 void launch_fused_step_tma(const FusedArgs &a, const FusedMaps &m, int *err, cudaStream_t st);
 void launch_wait_selftest(unsigned long long limit_ns, int *err, unsigned long long *elapsed_ns, cudaStream_t st);
+void launch_tile_wait_selftest(unsigned long long limit_ns, int *err, unsigned long long *elapsed_ns, cudaStream_t st);
+// bar: 0 before the launch
+void launch_mode_wait_selftest(unsigned long long limit_ns, unsigned *bar, int *err, unsigned long long *elapsed_ns,
+                               cudaStream_t st);
 
 // aux_kernels.cu
 void launch_mode_source(float *plane, const float *const ep_plane[3], const float *const mu_plane[3], int nx, int ny,

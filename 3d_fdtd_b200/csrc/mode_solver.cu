@@ -440,6 +440,14 @@ template <int EPT> __global__ void __launch_bounds__(kDotThreads) k_ms_krylov(Ms
     }
 }
 
+// the cycle's grid barrier with one arrival of two (fdtd_wait_selftest)
+__global__ void k_ms_wait_selftest(MsKrylov a, unsigned long long *elapsed_ns)
+{
+    const unsigned long long t0 = ms_clock();
+    ms_barrier(a, 2);
+    *elapsed_ns = ms_clock() - t0;
+}
+
 // y -= (*coef) x
 __global__ void k_ms_axpy(double2 *y, const double2 *x, const double2 *coef, int n2)
 {
@@ -901,6 +909,17 @@ struct Solver {
 };
 
 }  // namespace
+
+void launch_mode_wait_selftest(unsigned long long limit_ns, unsigned *bar, int *err, unsigned long long *elapsed_ns,
+                               cudaStream_t st)
+{
+    MsKrylov a{};
+    a.bar = bar;
+    a.err = err;
+    a.wait_ns = limit_ns;
+    note_launch();
+    k_ms_wait_selftest<<<1, 1, 0, st>>>(a, elapsed_ns);
+}
 
 bool mode_apply_beta2_device(const mode &in, double omega, mode &out)
 {

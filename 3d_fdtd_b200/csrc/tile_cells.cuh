@@ -96,7 +96,8 @@ __device__ __forceinline__ void tile_sync_init(TileSync *y)
 }
 constexpr unsigned long long kTileWaitNs = 1000000000ull;
 
-__device__ __forceinline__ bool tile_wait(TileSync *y, unsigned long long *bar, unsigned parity, bool after_abort = false)
+__device__ __forceinline__ bool tile_wait(TileSync *y, unsigned long long *bar, unsigned parity, bool after_abort = false,
+                                          unsigned long long limit_ns = kTileWaitNs)
 {
     const unsigned a = tile_s32(bar);
     unsigned long long t0 = 0;
@@ -111,7 +112,7 @@ __device__ __forceinline__ bool tile_wait(TileSync *y, unsigned long long *bar, 
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         if (!t0) t0 = now;
-        else if (now - t0 > kTileWaitNs) {
+        else if (now - t0 > limit_ns) {
             y->abort = 1;
             return false;
         }

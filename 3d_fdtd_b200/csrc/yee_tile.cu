@@ -452,6 +452,30 @@ void launch_yee_tile(const StreamArgs &a, const TileMaps *maps, const TileBox *t
     cudaLaunchKernelEx(&cfg, tile_kernel(a.L > 0, a.ca[0] != nullptr), a, maps, tiles, TileShape{p.tp, p.sw}, chain, err);
 }
 
+// a plane's wait for a copy that never comes (fdtd_wait_selftest): gives up, and the
+// next wait sees that at once
+__global__ void k_tile_wait_selftest(unsigned long long limit_ns, int *err, unsigned long long *elapsed_ns)
+{
+    __shared__ TileSync sync;
+    tile_sync_init(&sync);
+    __syncthreads();
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    const bool landed = tile_wait(&sync, &sync.full[0], 0, false, limit_ns);
+    __syncthreads();
+    const bool later = tile_wait(&sync, &sync.full[1], 0, false, limit_ns);
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    if (threadIdx.x != 0) return;
+    if (!landed && !later && *(volatile int *)&sync.abort) atomicExch(err, 1);
+    *elapsed_ns = t1 - t0;
+}
+
+void launch_tile_wait_selftest(unsigned long long limit_ns, int *err, unsigned long long *elapsed_ns, cudaStream_t st)
+{
+    note_launch();
+    k_tile_wait_selftest<<<1, 32, 0, st>>>(limit_ns, err, elapsed_ns);
+}
+
 }  // namespace fdtd
 
 // ---------------------------------------------------------------------------

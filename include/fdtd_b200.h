@@ -466,10 +466,11 @@ int timefield3d_checkpoint_load(timefield3d psi, const char *path);
 void fdtd_inject_allocation_failures(int n);
 
 /* Self-test of the engine's bounded device waits (no reference counterpart):
- * one block waits, with the routine the TMA pipeline uses, on a barrier that
- * nothing arrives on.  Expected result FDTD_ERR_TIMEOUT after about
- * limit_seconds (0 < limit <= 10), reported like a real pipeline timeout, with
- * the CUDA context still usable; *elapsed_seconds = the device-side wait. */
+ * one block each waits, with the routines of the fused step, of the streaming
+ * tiles and of the mode solver, for what never comes.  Expected result
+ * FDTD_ERR_TIMEOUT, each after about limit_seconds (0 < limit <= 10), reported
+ * like a real timeout, with the CUDA context still usable; *elapsed_seconds =
+ * the longest of the device-side waits. */
 int fdtd_wait_selftest(double limit_seconds, double *elapsed_seconds);
 /* Candidate sweep: advance `ngrids` grids together, grid i by nsteps[i] steps
  * (uneven counts allowed); returns at once, each grid's stream continues after
