@@ -289,8 +289,8 @@ struct TilePlan {
     double span = 0;             // estimate of the launch (us)
 };
 int tile_supported(int nx, int ny, int nz, bool lossy, int L);
-// tiles for a grid over nsm blocks; ty_cap > 0 caps the rows of a band
-bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out, int ty_cap = 0);
+// tiles for a grid over nsm blocks
+bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out);
 bool tile_configure(size_t smem, int threads);
 // TMA descriptors of one input set, in device memory
 struct TileMaps {

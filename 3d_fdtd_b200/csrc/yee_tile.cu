@@ -30,7 +30,6 @@
 namespace fdtd {
 
 constexpr int kTileMaxThreads = 512;
-constexpr size_t kTileSmemBudget = kStreamSmemBudget;
 
 // the units of a chain (StepChain), unit u by warp u / blocks of block u % blocks
 __device__ __forceinline__ void chain_units(const StepChain &c, int nx, int ny)
@@ -114,7 +113,7 @@ struct Columns {
 
 // a row split into nxt tiles of about equal threads (a slab quad has four), the
 // right halo quad of each but the last outside the x slabs; rows as many as fit
-bool columns_of(int nx, int L, bool lossy, int nxt, int ty_cap, Columns *out)
+bool columns_of(int nx, int L, bool lossy, int nxt, Columns *out)
 {
     const int QX = nx / 4;
     int QL = 0, QR = QX;
@@ -140,12 +139,12 @@ bool columns_of(int nx, int L, bool lossy, int nxt, int ty_cap, Columns *out)
     out->sw = 0;   // a halo quad at every cut
     for (int c = 0; c < nxt; c++) out->sw = std::max(out->sw, out->q[c + 1] - out->q[c] + (c > 0) + (c + 1 < nxt));
     out->tp = 0;
-    for (int tp = 2; tp <= (ty_cap > 0 ? ty_cap : 64) + 1; tp++) {
+    for (int tp = 2; tp <= 65; tp++) {
         int th = 0;
         for (int c = 0; c < nxt; c++) th = std::max(th, tile_roles(nx, L, out->q[c], out->q[c + 1], tp).threads);
         const TileShape sh{tp, out->sw};
         const size_t bytes = sh.floats(lossy, L) * sizeof(float);
-        if (th > kTileMaxThreads || !sh.fits(lossy) || bytes > kTileSmemBudget) break;
+        if (th > kTileMaxThreads || !sh.fits(lossy) || bytes > kStreamSmemBudget) break;
         out->tp = tp;
         out->threads = th;
         out->smem = bytes;
@@ -342,10 +341,10 @@ void plan_chunks(const ColumnSet &c, const std::vector<double> &weight, double w
 // rows in as few tiles as fit: a second tile a row costs more than the wider bands
 // save (200 cells without CPML, in halves: 159 us against 123), since its edges split
 // lines and DRAM bursts
-static bool tile_columns(int nx, int L, bool lossy, int ty_cap, Columns *col)
+static bool tile_columns(int nx, int L, bool lossy, Columns *col)
 {
     for (int nxt = 1; nxt <= 8; nxt++)
-        if (columns_of(nx, L, lossy, nxt, ty_cap, col)) return true;
+        if (columns_of(nx, L, lossy, nxt, col)) return true;
     return false;
 }
 
@@ -354,14 +353,14 @@ int tile_supported(int nx, int ny, int nz, bool lossy, int L)
     if (nx % 4 != 0 || nx < 8 || ny < 3 || nz < 3 || L < 0) return 0;
     if ((long long)nx * ny * nz >= (1LL << 31)) return 0;   // cell indices are 32-bit (sidx_t)
     Columns c;
-    return tile_columns(nx, L, lossy, 0, &c);
+    return tile_columns(nx, L, lossy, &c);
 }
 
-bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out, int ty_cap)
+bool tile_plan(int nx, int ny, int nz, int L, bool lossy, int nsm, TilePlan *out)
 {
-    if (!tile_supported(nx, ny, nz, lossy, L) || nsm <= 0 || ty_cap < 0) return false;
+    if (!tile_supported(nx, ny, nz, lossy, L) || nsm <= 0) return false;
     Columns col;
-    if (!tile_columns(nx, L, lossy, ty_cap, &col)) return false;
+    if (!tile_columns(nx, L, lossy, &col)) return false;
     std::vector<double> weight;
     double w = 0;
     for (int k = 1; k <= nz - 2; k++) {
