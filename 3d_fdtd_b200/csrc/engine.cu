@@ -1858,6 +1858,12 @@ TaperDev::~TaperDev()
     dfree(d_grad);
 }
 
+// an edge store's buffers change: graphs that hold their addresses are captured anew
+void drop_graphs()
+{
+    for (auto &kv : grid_table()) kv.second->version++;
+}
+
 TaperDev *taper_lookup(const adjoint3d_taper &t, bool create)
 {
     auto &tab = taper_table();
@@ -1896,6 +1902,7 @@ bool taper_prepare(TaperDev *td, const adjoint3d_taper &t, Grid *g)
     size_t es = g->prec == FDTD_F64 ? 8 : 4;
     if (resize) {
         cudaDeviceSynchronize();
+        drop_graphs();
         dfree(td->d_fwd);
         dfree(td->d_adj);
         dfree(td->d_cells);

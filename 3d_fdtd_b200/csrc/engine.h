@@ -276,6 +276,7 @@ struct TaperDev {
     ~TaperDev();
 };
 TaperDev *taper_lookup(const adjoint3d_taper &t, bool create);
+void drop_graphs();
 void taper_unregister(const adjoint3d_taper &t);
 bool taper_prepare(TaperDev *td, const adjoint3d_taper &t, Grid *g);
 bool enqueue_taper_store(TaperDev *td, Grid *g, int which, int t_index, const long long *d_step, int t0, int dir);

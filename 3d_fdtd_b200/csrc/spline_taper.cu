@@ -213,6 +213,7 @@ bool store_prepare(SplineStore *s, Grid *g)
     const int ncell = 6 * height * length;   // per (k, j, edge): the edge cell and its two x neighbours
     if (td->ncell != ncell || td->duration != s->duration || td->prec != g->prec) {
         cudaDeviceSynchronize();
+        drop_graphs();
         dfree(td->d_fwd); dfree(td->d_adj); dfree(td->d_cells); dfree(td->d_grad);
         td->ncell = ncell;
         td->duration = s->duration;
