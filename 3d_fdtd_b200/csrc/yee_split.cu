@@ -15,7 +15,7 @@
 // previous plane's stores (the arrays may alias), one memory latency a plane,
 // and a 64^3 grid had 128 blocks.  With a thread a cell the z and y neighbours
 // come from L2: FP64 steps of the 200 x 160 x 400 grid with a 12-cell CPML went
-// from 0.85 to 0.48 ms (the cells in no slab move 4.8 TB/s in E, 5.5 in H), and of
+// from 0.85 to 0.48 ms (the cells in no slab move 4.8 TB/s in E, 5.9 in H, the slabs' 3.7 and 3.9), and of
 // a 64^3 grid with the Mur boundary from 104 to 25 us (18 now).
 // FP64 divisions cost as much as a third of the traffic: a cell whose three
 // permittivities are equal (every rasteriser writes them so) takes its

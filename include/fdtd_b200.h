@@ -232,7 +232,8 @@ enum fdtd_precision { FDTD_F64 = 0, FDTD_F32 = 1 };
  * through its planes, E and H of a plane in one pass, reading each array once
  * and writing the other field set; nx % 4 == 0, fewer than 2^31 cells; one
  * kernel for grids whose E coefficients agree on a cell's components, one for the
- * others).  AUTO picks stream where the grid allows it, else flat4 where nx allows, else flat.  wave's fields are
+ * others; with a CPML, rows of over about 750 cells on fewer than 3.5 million cells
+ * go to flat4).  AUTO picks stream where the grid allows it, else flat4 where nx allows, else flat.  wave's fields are
  * bit-identical to flat4's; stream's agree with flat4's to float rounding. */
 enum fdtd_yee_variant {
     FDTD_YEE_AUTO = 0, FDTD_YEE_FLAT = 1, FDTD_YEE_FUSED = 2, FDTD_YEE_FLAT4 = 3, FDTD_YEE_WAVE = 4,
