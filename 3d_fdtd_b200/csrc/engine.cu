@@ -672,6 +672,9 @@ static bool build_profiles(Grid *g, double dt)
             }
         }
     }
+    // the streaming tiles fill their table of these before they wait for the launch
+    // before: on the device before any launch that reads them is enqueued
+    CK(cudaStreamSynchronize(g->st));
     g->prof_dt = dt;
     return true;
 }
@@ -801,6 +804,8 @@ static bool tile_prepare(Grid *g)
         }
     if (!dalloc(&g->d_maps, sizeof maps, g->st, false)) return false;
     CK(cudaMemcpyAsync(g->d_maps, maps, sizeof maps, cudaMemcpyHostToDevice, g->st));
+    // a block reads its box before it waits for the launch before (as build_profiles)
+    CK(cudaStreamSynchronize(g->st));
     std::copy(arrays, arrays + 14, g->maps_of);
     g->version++;
     return true;

@@ -60,3 +60,12 @@ def test_read_only_loads_take_only_what_no_step_writes():
             seen += 1
         assert "ld.global.nc" not in text
     assert seen > 10
+
+
+def test_tables_read_before_the_wait_are_uploaded_and_waited_for():
+    # a tile's block reads its box and the CPML profiles before it waits for the previous
+    # launch: the host waits for their copies before it enqueues any
+    text = source("engine.cu")
+    for f in ("bool build_profiles(Grid *g, double dt)", "bool tile_prepare(Grid *g)"):
+        b = body(text, text.index(f))
+        assert "cudaStreamSynchronize(g->st)" in b[b.rindex("cudaMemcpyAsync"):], f
