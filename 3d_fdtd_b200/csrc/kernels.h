@@ -110,8 +110,8 @@ struct TailArgs {
 // waits for any of it.  The step counter stands still until the chain's end.  A tail
 // launch between two steps is latency that nothing hides (a block of the step takes a
 // whole SM, so none of the tail's starts beside one): a step with two monitors of 11
-// frequencies and a source took 175 us on 200x160x400, 165 in a chain, 160 without
-// them; one with edge stores on 256x128x128 81 us, 75 in a chain.
+// frequencies and a source took 175 us on 200x160x400, 163 in a chain, 158 without
+// them; one with edge stores on 256x128x128 81 us, 73 in a chain.
 constexpr int kChainStores = 4;
 struct ChainStore {
     const long long *cells;

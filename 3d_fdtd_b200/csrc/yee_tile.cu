@@ -19,8 +19,8 @@
 //  - all columns are cut at the same planes, in one or two waves of blocks: tiles
 //    that run side by side read a shared halo row from DRAM once (kInStep below).
 // Per step, before (three coefficients, cp.async) and now: 200x160x400 with CPML 189
-// and 160 us (5.02 TB/s of algorithmic bytes), with PEC 144 and 115 us; 384x256x384
-// CPML 792 and 411; 256x128x128 CPML 77 and 69; 96x80x64 CPML, conductivity 45 and
+// and 158 us (5.07 TB/s of algorithmic bytes), with PEC 144 and 115 us; 384x256x384
+// CPML 792 and 405; 256x128x128 CPML 77 and 68; 96x80x64 CPML, conductivity 45 and
 // 14 us.  Two blocks an SM (96 registers) spill with CPML and gave nothing without.
 #include "tile_cells.cuh"
 #include "plane_ops.cuh"
@@ -314,7 +314,7 @@ void plan_chunks(const ColumnSet &c, const std::vector<double> &weight, double w
             acc += weight[q];
             // chunk i ends here; where as many planes are left as chunks, each is one
             // (a cut that was let pass there left all the rest to one chunk: 48x40x44
-            // with a 6-cell CPML had a tile of 19 planes and took 44.6 us, now 9.9)
+            // with a 6-cell CPML had a tile of 19 planes and took 44.6 us, now 9.7)
             const int i = (int)at.size(), spare = planes - q - 1 - (m - i);
             if (i < m && spare >= 0 && (spare == 0 || acc >= w * i / m - 0.5 * weight[q])) at.push_back(q + 1);
         }
